@@ -97,6 +97,20 @@ static bool encode_byte_map(CUtensorMap* map, const void* p, unsigned long long 
              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// The digit rows of one matrix, p[3][rows][K], as [K/128][3][rows][128 bytes]; one box =
+// [box_chunks][3][box_rows][128 bytes], 128-byte swizzle.
+static bool encode_digit_map(CUtensorMap* map, const void* p, unsigned long long rows, int K, int box_rows, int box_chunks) {
+  EncodeTiledFn enc = encode_tiled_fn();
+  if (!enc) return false;
+  const cuuint64_t gdim[4] = {128, cuuint64_t(rows), kDigits, cuuint64_t(K / 128)};
+  const cuuint64_t gstr[3] = {cuuint64_t(K), cuuint64_t(rows) * cuuint64_t(K), 128};
+  const cuuint32_t box[4] = {128, cuuint32_t(box_rows), kDigits, cuuint32_t(box_chunks)};
+  const cuuint32_t estr[4] = {1, 1, 1, 1};
+  return enc(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, const_cast<void*>(p), gdim, gstr, box, estr,
+             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 static bool encode_weight_map(CUtensorMap* map, const uint8_t* qt, int N, int K, int kc) {
   return encode_byte_map(map, qt, (unsigned long long)N, K, kTileRows, kc / 128);
 }
@@ -357,12 +371,16 @@ wkv_rows_kernel(int B, int T, int C, const float* __restrict__ w, const float* _
                 const float* __restrict__ v, const float* __restrict__ gate, float* __restrict__ aa,
                 float* __restrict__ bb, float* __restrict__ pp, long long state_stride) {
   griddep_launch_dependents();
-  griddep_wait();
   const int idx = blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= B * C) return;
   const int s = idx / C, c = idx - s * C;
-  const float wv = w[c], uv = u[c];
+  const float wv = __ldg(w + c), uv = __ldg(u + c);
   const size_t so = size_t(s) * state_stride + c;
+  // the state rows were last touched a whole step ago: on their way from DRAM while the GEMM in front still runs
+  asm volatile("prefetch.global.L2 [%0];" ::"l"(aa + so));
+  asm volatile("prefetch.global.L2 [%0];" ::"l"(bb + so));
+  asm volatile("prefetch.global.L2 [%0];" ::"l"(pp + so));
+  griddep_wait();
   float a = aa[so], q = bb[so], p = pp[so];
   const size_t base = size_t(s) * T * C + c;
   // The recurrence is sequential in t but its inputs are not: fetch eight steps at a time so the
@@ -525,19 +543,27 @@ static size_t gemm_workspace_bytes(int k_in, int nmat, int rows) {
 static thread_local bool g_chain_rows = true;   // set per call by forward_rows_impl / gemm_u8
 
 template <typename Kernel, typename... Args>
-static cudaError_t launch_chained(Kernel kernel, dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
-  if (!g_chain_rows) {
-    kernel<<<grid, block, smem, stream>>>(args...);
-    return cudaGetLastError();
-  }
+static cudaError_t launch_clustered(int cluster, Kernel kernel, dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
   cudaLaunchConfig_t cfg;
   memset(&cfg, 0, sizeof(cfg));
   cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr; cfg.numAttrs = 1;
+  cudaLaunchAttribute attr[2];
+  int n = 0;
+  if (g_chain_rows) {
+    attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[n++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  if (cluster > 1) {
+    attr[n].id = cudaLaunchAttributeClusterDimension;
+    attr[n].val.clusterDim.x = unsigned(cluster); attr[n].val.clusterDim.y = 1; attr[n++].val.clusterDim.z = 1;
+  }
+  cfg.attrs = attr; cfg.numAttrs = unsigned(n);
   return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
+template <typename Kernel, typename... Args>
+static cudaError_t launch_chained(Kernel kernel, dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
+  return launch_clustered(1, kernel, grid, block, smem, stream, args...);
 }
 
 template <int NT, int MODE, int G>
@@ -596,67 +622,92 @@ static cudaError_t launch_rows_prep(const RowsPrepParams& P_in, cudaStream_t str
   }
 }
 
-// Fills the tensor maps of P (weights and digit rows) and launches the tile GEMM.  digits: [nseg][3][Rpad][K].
-static cudaError_t launch_tile_gemm(GemmParams& P, const b200rwkv_matrix* const* mats, const signed char* digits,
-                                    cudaStream_t stream, const char** why) {
+// Encodes the tensor maps of P (weights and digit rows) for one tile shape and launches the tile GEMM.
+// digits: [nseg][3][Rpad][K].  kc = 0: chunks per stage by gemm_chunks_per_stage.
+static cudaError_t launch_tile_gemm_as(GemmParams& P, const b200rwkv_matrix* const* mats, const signed char* digits, bool pair, int Rt,
+                                       int ksplit, int kc, cudaStream_t stream, const char** why) {
   static bool configured[64];
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
   *why = "tile_gemm launch failed";
   if (dev >= 0 && dev < 64 && !configured[dev]) {
-    e = cudaFuncSetAttribute(tile_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemmSmem);
+    e = cudaFuncSetAttribute(tile_gemm_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemmSmem);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(tile_gemm_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemmSmem);
     if (e != cudaSuccess) return e;
     configured[dev] = true;
   }
-  // Tile shape.  The kernel is bound by operand bytes entering each SM (128 bytes of K per step for
-  // mt weight rows and 3*Rt digit rows) plus a fixed cost per tile; the launch takes as many rounds
-  // as the busiest CTA has tiles.  Few rows want small tiles (many CTAs, every weight byte still
-  // read once per row tile from L2); many rows want the 256 x 80 tile (most MACs per byte).
-  {
-    const long long sms = device_sms() > 0 ? device_sms() : 1;
-    const double fixed = 225.0 * 1024;   // ~3 us of a tile (start, accumulator hand-off, epilogue tail) in ingest bytes
-    const int nk = P.K / 128;
-    double best = 0.0;
-    P.mt = 128; P.Rt = 16; P.ksplit = 1;
-    for (int mt = 128; mt <= kGemmM; mt += 128) {
-      for (int rt = 16; rt <= kGemmRowsMax; rt += 16) {
-        long long tiles = 0;
-        for (int s = 0; s < P.nseg; ++s) tiles += (long long)((P.R + rt - 1) / rt) * ((P.seg[s].N + mt - 1) / mt);
-        for (int ks = 1; ks <= 8; ks *= 2) {
-          // K slices: only where the scratch exists and fits, and where they create CTAs the launch lacks
-          if (ks > 1 && (!P.sk_acc || mt != 128 || rt > kSplitMaxRt || tiles > kSplitMaxTiles || nk % ks != 0 ||
-                         nk / ks < 4 || tiles * (ks / 2) >= sms))
-            continue;
-          const double rounds = double((tiles * ks + sms - 1) / sms);
-          const double reduce = ks > 1 ? 2.0 * mt * kDigits * rt * 4 + 100.0 * 1024 : 0.0;   // atomics out, totals back, ticket
-          const double cost = rounds * (double(nk / ks) * 128.0 * (mt + kDigits * rt) + fixed + reduce);
-          if (best == 0.0 || cost < best) { best = cost; P.mt = mt; P.Rt = rt; P.ksplit = ks; }
-        }
-      }
-    }
-  }
+  P.pair = pair ? 1 : 0; P.Rt = Rt; P.ksplit = ksplit;
+  const int weight_rows = pair ? 2 * kGemmM : kGemmM, rows_tile = pair ? 2 * Rt : Rt;
+  P.dbuf = kDigits * rows_tile <= kGemmAcc1Col ? 1 : 0;
+  const int chunk = (kGemmM + kDigits * Rt) * 128, nk = P.K / 128 / ksplit;
+  P.kc = kc > 0 ? kc : gemm_chunks_per_stage(chunk, nk);
+  P.stage_bytes = P.kc * chunk;
+  P.stages = std::min(kGemmRingBytes / P.stage_bytes, kGemmMaxStages);
   for (int s = 0; s < P.nseg; ++s) {
     GemmSeg& S = P.seg[s];
-    if (!encode_byte_map(&S.wmap, mats[s]->qt, (unsigned long long)S.N, P.K, P.mt, 1) ||
-        !encode_byte_map(&S.xmap, digits + size_t(s) * kDigits * P.Rpad * P.K, (unsigned long long)kDigits * P.Rpad, P.K,
-                         P.Rt, 1)) {
+    if (!encode_byte_map(&S.wmap, mats[s]->qt, (unsigned long long)S.N, P.K, kGemmM, P.kc) ||
+        !encode_digit_map(&S.xmap, digits + size_t(s) * kDigits * P.Rpad * P.K, (unsigned long long)P.Rpad, P.K, Rt, P.kc)) {
       *why = "cuTensorMapEncodeTiled failed";
       return cudaErrorInvalidValue;
     }
   }
-  P.row_tiles = (P.R + P.Rt - 1) / P.Rt;
-  P.block_tiles = gemm_block_tiles(P.row_tiles, P.Rt, P.K);
+  P.row_tiles = (P.R + rows_tile - 1) / rows_tile;
+  P.block_tiles = gemm_block_tiles(P.row_tiles, rows_tile, P.K);
   P.ntiles = 0;
   for (int s = 0; s < P.nseg; ++s) {
-    P.tiles_seg[s] = P.row_tiles * ((P.seg[s].N + P.mt - 1) / P.mt);
+    P.tiles_seg[s] = P.row_tiles * ((P.seg[s].N + weight_rows - 1) / weight_rows);
     P.ntiles += P.tiles_seg[s];
   }
+  *why = "tile_gemm launch failed";
   const int items = P.ntiles * P.ksplit;
-  const dim3 grid(items < device_sms() ? items : device_sms());
-  return launch_chained(tile_gemm_kernel, grid, dim3(kGemmThreads), size_t(kGemmSmem), stream, P);
+  if (pair) {
+    const int pairs = items < device_sms() / 2 ? items : device_sms() / 2;
+    return launch_clustered(2, tile_gemm_kernel<true>, dim3(2 * pairs), dim3(kGemmThreads), size_t(kGemmSmem), stream, P);
+  }
+  return launch_chained(tile_gemm_kernel<false>, dim3(items < device_sms() ? items : device_sms()), dim3(kGemmThreads), size_t(kGemmSmem), stream, P);
 }
 
+// Tile shape of a launch: the cheapest of rounds of tiles x (K steps x time of a step + what a tile costs
+// besides).  The step times (128 bytes of K, us) are measured on launches of one round (7B ffn value,
+// K = 16384, 16 to 320 rows); they are shared-memory traffic (operands in by TMA, out to the tensor
+// core), which is why a pair, whose CTAs each hold half of the digit rows, needs less per row.  A tile
+// whose accumulator has no second buffer waits about 3 us for its epilogue; so does a K slice for its
+// atomics and ticket.
+static void gemm_pick_tile(const GemmParams& P, int* pair, int* Rt, int* ksplit) {
+  static const double step_single[5] = {0.19, 0.24, 0.335, 0.345, 0.37}, step_pair[5] = {0.22, 0.325, 0.40, 0.455, 0.565};   // Rt = 16, 32, .. 80
+  const long long sms = device_sms() > 1 ? device_sms() : 2;
+  const int nk = P.K / 128;
+  double best = 0.0;
+  for (int pr = 0; pr <= 1; ++pr) {
+    for (int i = 0; i < 5; ++i) {
+      const int rt = 16 * (i + 1), rows = pr ? 2 * rt : rt, wrows = pr ? 2 * kGemmM : kGemmM;
+      if (rt > 16 && rows - (pr ? 32 : 16) >= P.R) continue;     // a smaller tile holds all rows as well
+      const long long row_tiles = (P.R + rows - 1) / rows;
+      long long tiles = 0;
+      for (int s = 0; s < P.nseg; ++s) tiles += row_tiles * ((P.seg[s].N + wrows - 1) / wrows);
+      const bool dbuf = kDigits * rows <= kGemmAcc1Col;
+      for (int ks = 1; ks <= 8; ks *= 2) {
+        // K slices: only where the scratch exists and fits, and where they create CTAs the launch lacks
+        if (ks > 1 && (!P.sk_acc || pr || rt > kSplitMaxRt || tiles > kSplitMaxTiles || nk % ks != 0 || nk / ks < 4 ||
+                       tiles * (ks / 2) >= sms))
+          continue;
+        const long long units = pr ? sms / 2 : sms;
+        const double rounds = double((tiles * ks + units - 1) / units);
+        const double cost = rounds * (double(nk / ks) * (pr ? step_pair[i] : step_single[i]) + (ks > 1 || !dbuf ? 3.0 : 0.8));
+        if (best == 0.0 || cost < best) { best = cost; *pair = pr; *Rt = rt; *ksplit = ks; }
+      }
+    }
+  }
+}
+
+// Picks the tile shape and launches the tile GEMM.  digits: [nseg][3][Rpad][K].
+static cudaError_t launch_tile_gemm(GemmParams& P, const b200rwkv_matrix* const* mats, const signed char* digits,
+                                    cudaStream_t stream, const char** why) {
+  int pair = 0, Rt = 16, ksplit = 1;
+  gemm_pick_tile(P, &pair, &Rt, &ksplit);
+  return launch_tile_gemm_as(P, mats, digits, pair != 0, Rt, ksplit, 0, stream, why);
+}
 static void fill_gemm_seg(GemmSeg& s, const b200rwkv_matrix& m, const SegScalars* scal, float* out, long long ldo) {
   memset(&s, 0, sizeof(s));
   s.rx = m.rx; s.mx = m.mx; s.half = m.half; s.N = m.n_out; s.act = ACT_NONE;

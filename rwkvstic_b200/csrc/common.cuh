@@ -17,6 +17,18 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
+// Warp index as a value the compiler knows to be the same in all lanes, and one lane of a converged
+// warp.  Loops that issue TMA copies or tensor-core instructions run in all lanes of their warp, with
+// warp-uniform values, and only the instruction itself is issued by the elected lane: the operands of
+// these instructions live in uniform registers, and in a branch taken by one lane (`lane == 0`) every
+// one of them has to be moved there first, which bounded an MMA at 100 to 190 clocks whatever its size.
+__device__ __forceinline__ int warp_index() { return __shfl_sync(0xffffffffu, int(threadIdx.x >> 5), 0); }
+__device__ __forceinline__ bool elect_one() {
+  uint32_t ok;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok));
+  return ok != 0;
+}
+
 __device__ __forceinline__ unsigned long long globaltimer_ns() {
   unsigned long long t;
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
@@ -29,6 +41,14 @@ __device__ __forceinline__ unsigned long long globaltimer_ns() {
 // writes are visible; a no-op when the kernel was launched without the attribute.
 __device__ __forceinline__ void griddep_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// Ask L2 for n floats of constants, cooperatively by nt threads.  For kernels that wait on a launch
+// dependency and then read parameter vectors which the weight stream has long evicted: requested
+// before the wait, the DRAM latency is paid while the previous kernel still runs.
+__device__ __forceinline__ void prefetch_l2_floats(const float* p, int n, int tid, int nt) {
+  if (!p) return;
+  for (int i = tid * 32; i < n; i += nt * 32) asm volatile("prefetch.global.L2 [%0];" ::"l"(p + i));
+}
 
 // ---- mbarrier -----------------------------------------------------------------------------------
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {

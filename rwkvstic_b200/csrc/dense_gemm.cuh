@@ -25,9 +25,10 @@
 
 namespace b200 {
 
+constexpr int kDgM = 256;
 constexpr int kDgRowsMax = 240;                                  // activation rows per tile: 30 KB of a stage
-constexpr int kDgStageBytes = kGemmABytes + kDgRowsMax * 128;    // 62 KB
-constexpr int kDgRingBytes = kGemmStages * kDgStageBytes;          // 186 KB: three stages of the largest tile, up to eight of a small one
+constexpr int kDgStageBytes = (kDgM + kDgRowsMax) * 128;    // 62 KB
+constexpr int kDgRingBytes = 3 * kDgStageBytes;          // 186 KB: three stages of the largest tile, up to eight of a small one
 constexpr int kDgMaxStages = 8;                                  // barriers: full 0..7, empty 8..15
 constexpr int kDgSmem = kGemmOffRing + kDgRingBytes;
 constexpr int kDgSplitMaxItems = 640;                            // tiles x slices of a split launch (its tickets)
@@ -101,7 +102,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) dense_tile_gemm_kernel(const 
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem);
   const uint32_t full0 = smem_u32(bars), empty0 = smem_u32(bars + 8);
   const uint32_t acc_full0 = smem_u32(bars + 16), acc_empty0 = smem_u32(bars + 18);
-  const bool dbuf = P.mt != kGemmM;
+  const bool dbuf = P.mt != kDgM;
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + 256);
   volatile int* issued_ptr = reinterpret_cast<volatile int*>(smem + 260);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + 264);
@@ -127,25 +128,37 @@ __global__ void __launch_bounds__(kGemmThreads, 1) dense_tile_gemm_kernel(const 
   if (warp == 0) {
     // ---------------------------------------------------------------- TMA producer
     if (lane == 0) {
-      griddep_wait();   // the activation rows come from the kernel in front of this launch
       int issued = 0;
       bool ok = true;
+      // Weights are constants: the first ring of them is requested before the launch dependency resolves.
+      int early = 0;
+      for (int it = blockIdx.x; it < nitems_all && early < NS; it += gridDim.x) {
+        const DGemmTile T = dgemm_tile(P, it / S);
+        for (int kc = 0; kc < nk && early < NS; ++kc, ++early) {
+          mbar_arrive_expect_tx(full0 + 8 * early, a_bytes + b_bytes);
+          tma_load_3d(smem_u32(ring + size_t(early) * P.stage_bytes), &P.seg[T.seg].wmap, 0, T.n0, (it % S) * nk + kc, full0 + 8 * early);
+        }
+      }
+      *issued_ptr = early;
+      griddep_wait();   // the activation rows come from the kernel in front of this launch
       for (int it = blockIdx.x; it < nitems_all && ok; it += gridDim.x) {
         const DGemmTile T = dgemm_tile(P, it / S);
         const DGemmSeg& Sg = P.seg[T.seg];
         const int kbase = (it % S) * nk;
         for (int kc = 0; kc < nk; ++kc, ++issued) {
           const int slot = issued % NS;
-          const uint32_t phase = uint32_t(issued / NS) & 1u;
-          if (!mbar_wait_bounded(empty0 + 8 * slot, phase ^ 1u, abort_flag)) {
-            if (P.status) atomicOr(P.status, B200RWKV_STATUS_WAIT_EMPTY);
-            ok = false;
-            break;
-          }
           const uint32_t bar = full0 + 8 * slot;
           const uint32_t dst = smem_u32(ring + size_t(slot) * P.stage_bytes);
-          mbar_arrive_expect_tx(bar, a_bytes + b_bytes);
-          tma_load_3d(dst, &Sg.wmap, 0, T.n0, kbase + kc, bar);                    // rows past N are zero-filled
+          if (issued >= early) {
+            const uint32_t phase = uint32_t(issued / NS) & 1u;
+            if (!mbar_wait_bounded(empty0 + 8 * slot, phase ^ 1u, abort_flag)) {
+              if (P.status) atomicOr(P.status, B200RWKV_STATUS_WAIT_EMPTY);
+              ok = false;
+              break;
+            }
+            mbar_arrive_expect_tx(bar, a_bytes + b_bytes);
+            tma_load_3d(dst, &Sg.wmap, 0, T.n0, kbase + kc, bar);                    // rows past N are zero-filled
+          }
           tma_load_3d(dst + a_bytes, &Sg.xmap, 0, T.row0, kbase + kc, bar);    // rows past the buffer too
         }
       }
@@ -159,7 +172,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) dense_tile_gemm_kernel(const 
       int step = 0, iter = 0;
       for (int it = blockIdx.x; it < nitems_all && ok; it += gridDim.x, ++iter) {
         const DGemmTile T = dgemm_tile(P, it / S);
-        const bool two = P.mt == kGemmM && T.n0 + 128 < P.seg[T.seg].N;
+        const bool two = P.mt == kDgM && T.n0 + 128 < P.seg[T.seg].N;
         const int buf = dbuf ? (iter & 1) : 0, use = dbuf ? (iter >> 1) : iter;
         const uint32_t tacc = tmem + uint32_t(buf * kGemmAcc1Col);
         if (!mbar_wait_bounded(acc_empty0 + 8 * buf, uint32_t(use & 1) ^ 1u, abort_flag)) {
@@ -185,9 +198,9 @@ __global__ void __launch_bounds__(kGemmThreads, 1) dense_tile_gemm_kernel(const 
             umma_f16(tacc, ad0 + uint64_t(2 * k), bd + uint64_t(2 * k), idesc, acc);
             if (two) umma_f16(tmem + kGemmAcc1Col, ad1 + uint64_t(2 * k), bd + uint64_t(2 * k), idesc, acc);
           }
-          umma_commit(empty0 + 8 * slot);
+          umma_commit<false>(empty0 + 8 * slot);
         }
-        if (ok) umma_commit(acc_full0 + 8 * buf);
+        if (ok) umma_commit<false>(acc_full0 + 8 * buf);
       }
     }
   } else if (warp >= 4) {
@@ -204,7 +217,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) dense_tile_gemm_kernel(const 
       const DGemmTile T = dgemm_tile(P, tile);
       const DGemmSeg& Sg = P.seg[T.seg];
       const int n0 = T.n0, row0 = T.row0;
-      const bool two = P.mt == kGemmM && n0 + 128 < Sg.N;
+      const bool two = P.mt == kDgM && n0 + 128 < Sg.N;
       const int buf = dbuf ? (iter & 1) : 0, use = dbuf ? (iter >> 1) : iter;
       const uint32_t acc_empty = acc_empty0 + 8 * buf;
       ok = __all_sync(0xffffffffu, mbar_wait_bounded(acc_full0 + 8 * buf, uint32_t(use & 1), abort_flag));
@@ -362,8 +375,13 @@ dense_rows_prep_kernel(const DRowsPrepParams P) {
   extern __shared__ __align__(16) float rp_smem[];      // [2][D]
   __shared__ float red[8];
   griddep_launch_dependents();
-  griddep_wait();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, D = P.D, D4 = P.D >> 2;
+  if (blockIdx.x == 0) {
+    prefetch_l2_floats(P.ln_w, D, tid, 256);
+    prefetch_l2_floats(P.ln_b, D, tid, 256);
+    for (int m = 0; m < P.nmix; ++m) prefetch_l2_floats(P.mix[m], D, tid, 256);
+  }
+  griddep_wait();
   auto block_sum = [&](float v) -> float {
     v = warp_sum(v);
     __syncthreads();

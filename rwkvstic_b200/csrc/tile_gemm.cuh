@@ -8,22 +8,27 @@
 // with the uint8 weights are exact integer sums recombined in int64.  Here the digit rows are the
 // B operand of 5th-generation tensor-core MMAs (tcgen05.mma kind::i8, u8 x s8 -> s32):
 //
-//   A  = mt weight rows    x 128 bytes of K   (one TMA box of qt[N][K], 128-byte swizzle, K-major; mt = 128 or 256)
-//   B  = 3*Rt digit rows   x 128 bytes of K   (three TMA boxes, [digit][Rt activation rows], Rt = 16..80)
-//   D  = 128 lanes x 3*Rt int32 columns per 128 weight rows in tensor memory (TMEM),
-//        column = digit*Rt + row.  A 256-row tile keeps its second accumulator at column 256 (two
-//        weight sub-tiles share one digit tile); with 128-row tiles columns 0 and 256 are two
-//        buffers, so the epilogue of one tile runs under the MMAs of the next.
+//   A  = 128 weight rows   x 128 bytes of K   (a TMA box of qt[N][K], 128-byte swizzle, K-major)
+//   B  = 3*Rt digit rows   x 128 bytes of K   (a TMA box [3 digits][Rt activation rows], Rt = 16..80)
+//   D  = 128 lanes x digit-row columns, int32, in tensor memory (TMEM)
 //
-// Persistent kernel, one CTA per SM looping over tiles; a CTA walks K in 128-byte steps through a
-// ring of shared-memory stages that runs on across tiles: warp 0 issues the TMA copies, warp 1
-// issues the MMAs (one elected thread; completion is signalled to the ring by tcgen05.commit on the
-// stage's mbarrier), warps 4-19 read the accumulators with tcgen05.ld and apply the affine terms
-// and the fused element-wise op.  The kernel is bound by operand traffic from L2 to shared memory
-// (int8 MMAs need ~250 MACs per byte to saturate, the 256 x 240 tile gives M*N/(M+N) = 124) until
-// the tensor pipe saturates (81 % active on the largest shapes).  Tiles that share a weight tile
-// are adjacent in issue order so it is read from HBM once and from L2 afterwards.  The host picks
-// mt, Rt and, for launches with too few tiles, a split of K over several CTAs (see GemmParams).
+// Two forms of one kernel.  Single: a CTA works on a tile of 128 weight rows x Rt activation rows.
+// Pair: the two CTAs of a cluster work on 256 weight rows x 2*Rt activation rows with
+// tcgen05.mma.cta_group::2; each holds half of the weight rows and half of the digit rows, the tensor
+// cores of both read both halves of the digit rows, and each CTA gets the accumulators of its own
+// weight rows, so the digit rows enter shared memory once per 256 weight rows instead of once per 128.
+//
+// Persistent kernel, one CTA per SM looping over tiles; a CTA walks K through a ring of shared-memory
+// stages that runs on across tiles: warp 0 issues the TMA copies, warp 1 issues the MMAs (one elected
+// lane; completion is signalled to the ring by tcgen05.commit on the stage's mbarrier), warps 4-19
+// read the accumulators with tcgen05.ld and apply the affine terms and the fused element-wise op.
+// What bounds it: shared-memory traffic.  A K step writes (128 + 3*Rt) * 128 bytes by TMA and the MMAs
+// read every operand row again per 32 bytes of K.  Measured (7B ffn value, K = 16384, per K step and
+// CTA): single 80 rows 0.37 us, pair 160 rows 0.565 us, the MMAs alone 0.26 and 0.51 us at 1.87 GHz.
+// L2 is not the limit (TMA boxes come from L2 at 16 to 19 TB/s in aggregate, 110 to 130 GB/s per SM).
+// Tiles that share a weight tile are adjacent in issue order so it is read from HBM once and from L2
+// afterwards.  The host picks the form, Rt and, for launches with too few tiles, a split of K over
+// several CTAs (see GemmParams).
 //
 // Every wait is bounded (common.cuh): on expiry the CTA raises its abort flag, sets a status bit,
 // skips its remaining work, and still frees its tensor memory before it retires.
@@ -33,12 +38,11 @@
 
 namespace b200 {
 
-constexpr int kGemmM = 256;                              // weight rows per tile = two MMA M=128 sub-tiles
-constexpr int kGemmRowsMax = 80;                         // activation rows per tile (multiple of 16)
+constexpr int kGemmM = 128;                              // weight rows a CTA holds of a tile
+constexpr int kGemmRowsMax = 80;                         // activation rows a CTA holds of a tile (multiple of 16)
 constexpr int kDigits = 3;
-constexpr int kGemmStages = 3;
-constexpr int kGemmABytes = kGemmM * 128;                // 32 KB
-constexpr int kGemmStageBytes = kGemmABytes + kDigits * kGemmRowsMax * 128;   // 62 KB
+constexpr int kGemmMaxStages = 8;                        // ring depth at most (barriers: full 0..7, empty 8..15)
+constexpr int kGemmRingBytes = 186 * 1024;
 constexpr int kGemmTmemCols = 512;                       // both accumulators; one CTA per SM (shared memory)
 constexpr int kGemmAcc1Col = 256;                        // first column of the second accumulator
 constexpr int kGemmEpiWarps = 16;                        // four per TMEM lane quadrant
@@ -51,7 +55,7 @@ constexpr int kSplitMaxRt = 32;                          // and its tile height
 constexpr size_t kSplitAccBytes = size_t(kSplitMaxTiles) * kDigits * kSplitMaxRt * 128 * 4;   // 15.7 MB
 constexpr int kGemmOffScal = 1024;                       // SegScalars[80]
 constexpr int kGemmOffRing = 4096;
-constexpr int kGemmSmem = kGemmOffRing + kGemmStages * kGemmStageBytes;
+constexpr int kGemmSmem = kGemmOffRing + kGemmRingBytes;
 
 // The digit rows of a launch are laid out [matrix][digit][Rpad][K] with Rpad = R rounded up to 16,
 // whatever tile height the GEMM then picks: a tile that reaches past row R reads the next digit
@@ -59,8 +63,8 @@ constexpr int kGemmSmem = kGemmOffRing + kGemmStages * kGemmStageBytes;
 inline int gemm_padded_rows(int R) { return (R + 15) / 16 * 16; }
 
 struct GemmSeg {
-  CUtensorMap wmap;    // u8 qt as [K/128][N][128 B], box [1][mt][128], 128-byte swizzle
-  CUtensorMap xmap;    // s8 digits as [K/128][3*Rpad][128 B], box [1][Rt][128], 128-byte swizzle
+  CUtensorMap wmap;    // u8 qt as [K/128][N][128 B], box [kc][128][128], 128-byte swizzle
+  CUtensorMap xmap;    // s8 digits as [K/128][3][Rpad][128 B], box [kc][3][Rt][128], 128-byte swizzle
   const float* rx;     // [N] or null
   const float* mx;     // [N] or null
   const SegScalars* scal;  // [R] per activation row: sd, zp, sumxs, sumx
@@ -76,21 +80,31 @@ struct GemmSeg {
 struct GemmParams {
   GemmSeg seg[kMaxSeg];
   int nseg, K, R, Rpad;
-  int Rt;              // activation rows per tile (multiple of 16, <= 80)
-  int mt;              // weight rows per tile: 256 (two accumulators) or 128 (small grids: more CTAs)
-  int row_tiles;       // ceil(R / Rt)
+  int Rt;              // activation rows one CTA holds of a tile (multiple of 16, <= 80)
+  int pair;            // tiles of a CTA pair: 256 weight rows x 2*Rt activation rows
+  int dbuf;            // the accumulator has two buffers
+  int kc;              // 128-byte chunks of K per stage (one TMA copy each for the weights and the digits of a stage)
+  int stages;          // ring depth
+  int stage_bytes;     // kc * (128 + 3*Rt) * 128, a multiple of 1024
+  int row_tiles;       // ceil(R / activation rows per tile)
   int block_tiles;     // row tiles per row block (tile order below); row_tiles when all digit rows fit L2 at once
-  int tiles_seg[kMaxSeg];  // tiles per matrix = row_tiles * ceil(N / mt)
+  int tiles_seg[kMaxSeg];  // tiles per matrix = row_tiles * ceil(N / weight rows per tile)
   int ntiles;          // all tiles of the launch; the grid is min(ntiles * ksplit, SMs), CTAs loop over work items
   // Split-K for launches with few tiles (few activation rows): work item = (tile, K slice); every
   // slice adds its int32 digit sums into sk_acc with integer atomics (exact, order-free), takes a
   // ticket, and the CTA that draws the last ticket of a tile reads the totals, runs the epilogue and
   // leaves sk_acc / sk_count zero again.  Nobody waits for anybody.
-  int ksplit;          // 1, 2, 4 or 8 slices (divides K/128; only with 128-row tiles and Rt <= 32)
+  int ksplit;          // 1, 2, 4 or 8 slices (divides K/128; only single-CTA tiles with Rt <= 32)
   int* sk_acc;         // [kSplitMaxTiles][3*Rt][128] int32, zero between launches
   unsigned* sk_count;  // [kSplitMaxTiles] tickets, zero between launches
   int* status;
 };
+
+__device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap* map, int c0, int c1, int c2, int c3, uint32_t bar) {
+  asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];" ::"r"(dst),
+               "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(bar)
+               : "memory");
+}
 
 // ---- tcgen05 wrappers ------------------------------------------------------------------------------
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
@@ -113,17 +127,83 @@ __host__ __device__ constexpr uint32_t umma_idesc_u8s8(int M, int N) {
   return (2u << 4) | (0u << 7) | (1u << 10) | (uint32_t(N >> 3) << 17) | (uint32_t(M >> 4) << 24);
 }
 
+template <bool kPair>
 __device__ __forceinline__ void umma_i8(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
-      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
+  if constexpr (kPair)
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::i8 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
+        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        : "memory");
+  else
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
+        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        : "memory");
 }
 
-// The mbarrier receives one arrival when every MMA issued so far by this thread has finished.
+// The mbarrier (in a pair: the one at this offset in either CTA) receives one arrival when every MMA
+// issued so far by this thread has finished.
+template <bool kPair>
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+  if constexpr (kPair)
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar), "h"((unsigned short)3)
+                 : "memory");
+  else
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+}
+
+// ---- CTA pairs (clusters of two) ---------------------------------------------------------------------
+__device__ __forceinline__ uint32_t cluster_ctarank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+// The even CTA's shared memory at the offset of `addr`, as a shared::cluster address.
+__device__ __forceinline__ uint32_t leader_addr(uint32_t addr) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(r) : "r"(addr));
+  return r;
+}
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// One arrival on the even CTA's barrier at this offset.
+__device__ __forceinline__ void mbar_arrive_leader(uint32_t bar) {
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(leader_addr(bar)) : "memory");
+}
+template <bool kPair>
+__device__ __forceinline__ void tmem_alloc(uint32_t slot) {
+  if constexpr (kPair) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(slot), "r"(kGemmTmemCols) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+  } else {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(slot), "r"(kGemmTmemCols) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+}
+template <bool kPair>
+__device__ __forceinline__ void tmem_dealloc(uint32_t tmem) {
+  if constexpr (kPair) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kGemmTmemCols) : "memory");
+  else asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kGemmTmemCols) : "memory");
+}
+// Operand copies into this CTA's shared memory; in a pair `bar` may be the other CTA's barrier.
+template <bool kPair>
+__device__ __forceinline__ void tma_operand_3d(uint32_t dst, const CUtensorMap* map, int c0, int c1, int c2, uint32_t bar) {
+  if constexpr (kPair)
+    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.cta_group::2 [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(dst),
+                 "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(bar)
+                 : "memory");
+  else tma_load_3d(dst, map, c0, c1, c2, bar);
+}
+template <bool kPair>
+__device__ __forceinline__ void tma_operand_4d(uint32_t dst, const CUtensorMap* map, int c0, int c1, int c2, int c3, uint32_t bar) {
+  if constexpr (kPair)
+    asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.cta_group::2 [%0], [%1, {%2, %3, %4, %5}], [%6];" ::"r"(dst),
+                 "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(bar)
+                 : "memory");
+  else tma_load_4d(dst, map, c0, c1, c2, c3, bar);
 }
 
 // 16 consecutive int32 columns of this warp's 32 lanes.
@@ -144,6 +224,13 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, int (&v)[8]) {
 }
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
+// A whole warp waits for a barrier; false (with the status bit set) when the bounded wait expired.
+__device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status, int bit) {
+  const bool ok = __all_sync(0xffffffffu, mbar_wait_bounded(bar, parity, abort_flag));
+  if (!ok && status && elect_one()) atomicOr(status, bit);
+  return ok;
+}
+
 // Tile t of a launch -> (segment, first weight row, first activation row).  Within a matrix the order is
 // row block, weight tile, row tile of the block: the CTAs working side by side share a weight tile, and
 // all weight tiles sweep over one block of digit rows (sized by the launcher to stay in L2) before the
@@ -158,126 +245,155 @@ __device__ __forceinline__ GemmTile gemm_tile(const GemmParams& P, int t) {
   const int nb = min(P.block_tiles, P.row_tiles - first);     // row tiles of this (maybe last, shorter) block
   const int idx = t - blk * per_block;
   const int wt = idx / nb;
-  return {s, wt * P.mt, (first + idx - wt * nb) * P.Rt};
+  return {s, P.pair ? wt * 256 : wt * 128, (first + idx - wt * nb) * (P.pair ? 2 * P.Rt : P.Rt)};
 }
 
 // Row tiles per block: three digit planes of a block's rows take at most kGemmDigitBlockBytes.
 constexpr long long kGemmDigitBlockBytes = 16ll << 20;   // measured best of 8 / 16 / 24 / 32 / 48 MB on the 126 MB L2
-inline int gemm_block_tiles(int row_tiles, int Rt, int K) {
-  const long long per_tile = (long long)kDigits * Rt * K;
+inline int gemm_block_tiles(int row_tiles, int rows_tile, int K) {
+  const long long per_tile = (long long)kDigits * rows_tile * K;
   const long long fit = per_tile > 0 ? kGemmDigitBlockBytes / per_tile : row_tiles;
   return int(fit < 1 ? 1 : fit > row_tiles ? row_tiles : fit);
 }
 
+// 128-byte K chunks per stage.  One turn of the producer and of the MMA issuer (wait, copies or MMAs,
+// commit) costs about 0.2 us whatever it moves, so small tiles take two chunks per turn, where three
+// stages of them still fit the ring (two stages are slower than twice as many half as large).
+inline int gemm_chunks_per_stage(int chunk_bytes, int nk) { return nk >= 2 && 3 * 2 * chunk_bytes <= kGemmRingBytes ? 2 : 1; }
+
+// kPair: two CTAs of a cluster work on one tile with tcgen05.mma.cta_group::2 (see the file comment).
+template <bool kPair>
 __global__ void __launch_bounds__(kGemmThreads, 1) tile_gemm_kernel(const __grid_constant__ GemmParams P) {
   extern __shared__ __align__(1024) unsigned char smem[];
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = warp_index(), lane = tid & 31;
   const int Rt = P.Rt;
   const int S = P.ksplit;
   const int nk = P.K / 128 / S;          // K steps of one work item
   const int nitems_all = P.ntiles * S;
-  const uint32_t a_bytes = uint32_t(P.mt) * 128u;
-  const uint32_t b_bytes = uint32_t(kDigits * Rt * 128);
-
+  const int rank = kPair ? int(cluster_ctarank()) : 0;                    // which half of the tile this CTA holds
+  const int first_item = kPair ? int(blockIdx.x >> 1) : int(blockIdx.x), item_stride = kPair ? int(gridDim.x >> 1) : int(gridDim.x);
+  const int KC = P.kc;
+  const uint32_t a_chunk = 128u * 128u, b_chunk = uint32_t(kDigits * Rt * 128);
+  const uint32_t a_bytes = uint32_t(KC) * a_chunk;      // a stage: KC weight chunks, then KC digit chunks
+  const int NS = P.stages;
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem);
   const uint32_t full0 = smem_u32(bars), empty0 = smem_u32(bars + 8);
   const uint32_t acc_full0 = smem_u32(bars + 16), acc_empty0 = smem_u32(bars + 18);   // two of each (8 bytes apart)
-  // With 128-row tiles one accumulator needs 3*Rt <= 240 columns, so two fit in TMEM: tile i+1 is
-  // accumulated at column 256 while the epilogue still reads tile i at column 0.  With 256-row tiles
-  // the second accumulator of the SAME tile lives at column 256 and tiles alternate on one buffer.
-  const bool dbuf = P.mt != kGemmM;
+  // An accumulator that fits 256 columns has two buffers, columns 0 and 256: the next tile is accumulated
+  // in one while the epilogue still reads the other.  A wider one (pair tiles of more than 80 rows) has
+  // one buffer of two parts: the first min(3*Rt, 128) digit rows of either CTA at column 0, the rest at 256.
+  const bool dbuf = P.dbuf != 0;
+  const int nb = kDigits * Rt, nb1 = kPair && nb > 128 ? 128 : nb;
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + 256);
   volatile int* issued_ptr = reinterpret_cast<volatile int*>(smem + 260);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + 264);
-  SegScalars* scal = reinterpret_cast<SegScalars*>(smem + kGemmOffScal);
+  float* scal = reinterpret_cast<float*>(smem + kGemmOffScal);      // [rows of the tile][4]: sd, zp, sumxs, sumx
   unsigned char* ring = smem + kGemmOffRing;
 
   if (tid == 0) {
-    for (int i = 0; i < kGemmStages; ++i) { mbar_init(full0 + 8 * i, 1); mbar_init(empty0 + 8 * i, 1); }
-    for (int i = 0; i < 2; ++i) { mbar_init(acc_full0 + 8 * i, 1); mbar_init(acc_empty0 + 8 * i, kGemmEpiWarps); }
+    for (int i = 0; i < kGemmMaxStages; ++i) { mbar_init(full0 + 8 * i, 1); mbar_init(empty0 + 8 * i, 1); }
+    for (int i = 0; i < 2; ++i) { mbar_init(acc_full0 + 8 * i, 1); mbar_init(acc_empty0 + 8 * i, (kPair ? 2 : 1) * kGemmEpiWarps); }
     *abort_flag = 0;
     *issued_ptr = 0;
     fence_mbar_init();
   }
-  if (warp == 2) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(kGemmTmemCols) : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-  }
+  if (warp == 2) tmem_alloc<kPair>(smem_u32(tmem_slot));
   tc_fence_before();
   __syncthreads();
+  if (kPair) cluster_sync();             // the partner's barriers exist before anything arrives on them
   tc_fence_after();
-  const uint32_t tmem = *tmem_slot;
+  const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
   griddep_launch_dependents();
 
-  // Persistent: CTA c handles tiles c, c + grid, c + 2*grid, ...  The operand ring runs on across
-  // tiles (the producer is already fetching the next tile while the epilogue of this one runs).
+  // Persistent: CTA (pair) c handles work items c, c + grid, c + 2*grid, ...  The operand ring runs on
+  // across tiles (the producer is already fetching the next tile while the epilogue of this one runs).
   if (warp == 0) {
-    // ---------------------------------------------------------------- TMA producer
-    if (lane == 0) {
-      griddep_wait();   // the digit rows come from the preparation kernel in front of this launch
-      int issued = 0;
-      bool ok = true;
-      for (int it = blockIdx.x; it < nitems_all && ok; it += gridDim.x) {
-        const GemmTile T = gemm_tile(P, it / S);
-        const GemmSeg& Sg = P.seg[T.seg];
-        const int kbase = (it % S) * nk;
-        for (int kc = 0; kc < nk; ++kc, ++issued) {
-          const int slot = issued % kGemmStages;
-          const uint32_t phase = uint32_t(issued / kGemmStages) & 1u;
-          if (!mbar_wait_bounded(empty0 + 8 * slot, phase ^ 1u, abort_flag)) {
-            if (P.status) atomicOr(P.status, B200RWKV_STATUS_WAIT_EMPTY);
-            ok = false;
-            break;
-          }
-          const uint32_t bar = full0 + 8 * slot;
-          const uint32_t dst = smem_u32(ring + size_t(slot) * kGemmStageBytes);
-          mbar_arrive_expect_tx(bar, a_bytes + b_bytes);
-          tma_load_3d(dst, &Sg.wmap, 0, T.n0, kbase + kc, bar);   // rows past N are zero-filled
-#pragma unroll
-          for (int d = 0; d < kDigits; ++d)
-            tma_load_3d(dst + kGemmABytes + uint32_t(d * Rt * 128), &Sg.xmap, 0, d * P.Rpad + T.row0, kbase + kc, bar);
+    // ---------------------------------------------------------------- TMA producer.  In a pair each CTA
+    // copies its own weight rows and its own half of the digit rows; both count their bytes on the
+    // even CTA's barrier, which is where the MMA issuer waits.
+    {
+      const uint32_t ring0 = smem_u32(ring), stage_bytes = uint32_t(P.stage_bytes);
+      const uint32_t full_at = kPair ? leader_addr(full0) : full0;
+      const uint32_t tx_bytes = kPair ? 2u * stage_bytes : stage_bytes;
+      // Weights are constants: the first ring of them is requested before the launch dependency
+      // resolves, while the preparation kernel in front of this launch still runs.  (An L2 prefetch of
+      // 64 to 512 KB per CTA beyond the ring was no faster at any size, 5 % slower at few rows.)
+      struct Cursor { int it, k0; GemmTile T; };
+      auto start = [&](Cursor& c) { c.it = first_item; c.k0 = 0; if (c.it < nitems_all) c.T = gemm_tile(P, c.it / S); };
+      auto next = [&](Cursor& c) {
+        if ((c.k0 += KC) >= nk) {
+          c.k0 = 0;
+          if ((c.it += item_stride) < nitems_all) c.T = gemm_tile(P, c.it / S);
         }
+      };
+      auto kstep = [&](const Cursor& c) { return (S == 1 ? 0 : (c.it % S) * nk) + c.k0; };
+      Cursor ld;
+      start(ld);
+      int early = 0;
+      for (; early < NS && ld.it < nitems_all; ++early, next(ld)) {
+        if (elect_one()) {
+          if (rank == 0) mbar_arrive_expect_tx(full0 + 8 * early, tx_bytes);
+          tma_operand_3d<kPair>(ring0 + uint32_t(early) * stage_bytes, &P.seg[ld.T.seg].wmap, 0, ld.T.n0 + rank * 128, kstep(ld), full_at + 8 * early);
+        }
+      }
+      *issued_ptr = early;
+      griddep_wait();   // the digit rows come from the preparation kernel in front of this launch
+      int issued = 0, slot = 0;
+      uint32_t phase = 0;
+      for (start(ld); ld.it < nitems_all; next(ld)) {
+        const GemmSeg& Sg = P.seg[ld.T.seg];
+        const uint32_t bar = full_at + 8 * slot, dst = ring0 + uint32_t(slot) * stage_bytes;
+        if (issued >= early) {
+          if (!warp_wait(empty0 + 8 * slot, phase ^ 1u, abort_flag, P.status, B200RWKV_STATUS_WAIT_EMPTY)) break;
+          if (elect_one()) {
+            if (rank == 0) mbar_arrive_expect_tx(full0 + 8 * slot, tx_bytes);
+            tma_operand_3d<kPair>(dst, &Sg.wmap, 0, ld.T.n0 + rank * 128, kstep(ld), bar);   // rows past N and chunks past K are zero-filled
+          }
+        }
+        if (elect_one()) tma_operand_4d<kPair>(dst + a_bytes, &Sg.xmap, 0, ld.T.row0 + rank * Rt, 0, kstep(ld), bar);
+        ++issued;
+        if (++slot == NS) { slot = 0; phase ^= 1u; }
       }
       *issued_ptr = issued;
     }
   } else if (warp == 1) {
-    // ---------------------------------------------------------------- MMA issuer
-    if (lane == 0) {
-      const uint32_t idesc = umma_idesc_u8s8(128, kDigits * Rt);
+    // ---------------------------------------------------------------- MMA issuer (the even CTA's, for both)
+    if (rank == 0) {
+      const uint32_t idesc1 = umma_idesc_u8s8(kPair ? 256 : 128, kPair ? 2 * nb1 : nb);
+      const uint32_t idesc2 = umma_idesc_u8s8(256, 2 * (nb - nb1));       // second part, if any (pair only)
+      const bool second = kPair && nb > nb1;
+      const uint32_t ring0 = smem_u32(ring), stage_bytes = uint32_t(P.stage_bytes);
       bool ok = true;
-      int step = 0, iter = 0;
-      for (int it = blockIdx.x; it < nitems_all && ok; it += gridDim.x, ++iter) {
-        const GemmTile T = gemm_tile(P, it / S);
-        const bool two = P.mt == kGemmM && T.n0 + 128 < P.seg[T.seg].N;   // second 128-row sub-tile holds real rows
+      int iter = 0, slot = 0;
+      uint32_t phase = 0;
+      for (int it = first_item; it < nitems_all && ok; it += item_stride, ++iter) {
         // the epilogue must have read this buffer's previous tile out of TMEM
         const int buf = dbuf ? (iter & 1) : 0, use = dbuf ? (iter >> 1) : iter;
         const uint32_t tacc = tmem + uint32_t(buf * kGemmAcc1Col);
-        if (!mbar_wait_bounded(acc_empty0 + 8 * buf, uint32_t(use & 1) ^ 1u, abort_flag)) {
-          if (P.status) atomicOr(P.status, B200RWKV_STATUS_WAIT_EMPTY);
-          ok = false;
-          break;
-        }
-        tc_fence_after();
-        for (int kc = 0; kc < nk; ++kc, ++step) {
-          const int slot = step % kGemmStages;
-          const uint32_t phase = uint32_t(step / kGemmStages) & 1u;
-          if (!mbar_wait_bounded(full0 + 8 * slot, phase, abort_flag)) {
-            if (P.status) atomicOr(P.status, B200RWKV_STATUS_WAIT_FULL);
-            ok = false;
-            break;
-          }
-          tc_fence_after();
-          const uint32_t a = smem_u32(ring + size_t(slot) * kGemmStageBytes);
-          const uint64_t ad0 = umma_desc(a), ad1 = umma_desc(a + 128 * 128), bd = umma_desc(a + kGemmABytes);
+        if (!warp_wait(acc_empty0 + 8 * buf, uint32_t(use & 1) ^ 1u, abort_flag, P.status, B200RWKV_STATUS_WAIT_EMPTY)) { ok = false; break; }
+        uint32_t acc = 0u;    // the first MMA of a tile overwrites the accumulator
+        for (int k0 = 0; k0 < nk; k0 += KC) {
+          if (!warp_wait(full0 + 8 * slot, phase, abort_flag, P.status, B200RWKV_STATUS_WAIT_FULL)) { ok = false; break; }
+          if (elect_one()) {
+            tc_fence_after();
+            const uint32_t a = ring0 + uint32_t(slot) * stage_bytes;
+            uint64_t ad = umma_desc(a), bd = umma_desc(a + a_bytes);
+            const int nc = min(KC, nk - k0);
+            for (int c = 0; c < nc; ++c) {
 #pragma unroll
-          for (int k = 0; k < 4; ++k) {   // 32 bytes of K per instruction: +2 in the descriptors' 16-byte address units
-            const uint32_t acc = (kc | k) != 0 ? 1u : 0u;
-            umma_i8(tacc, ad0 + uint64_t(2 * k), bd + uint64_t(2 * k), idesc, acc);
-            if (two) umma_i8(tmem + kGemmAcc1Col, ad1 + uint64_t(2 * k), bd + uint64_t(2 * k), idesc, acc);
+              for (int k = 0; k < 4; ++k) {   // 32 bytes of K per instruction: +2 in the descriptors' 16-byte address units
+                umma_i8<kPair>(tacc, ad + uint64_t(2 * k), bd + uint64_t(2 * k), idesc1, k == 0 && c == 0 ? acc : 1u);
+                if (second)
+                  umma_i8<kPair>(tmem + kGemmAcc1Col, ad + uint64_t(2 * k), bd + uint64_t(128 * 128 / 16 + 2 * k), idesc2, k == 0 && c == 0 ? acc : 1u);
+              }
+              ad += uint64_t(a_chunk >> 4); bd += uint64_t(b_chunk >> 4);
+            }
+            umma_commit<kPair>(empty0 + 8 * slot);             // frees the stage (in both CTAs) once these MMAs have read it
+            if (k0 + KC >= nk) umma_commit<kPair>(acc_full0 + 8 * buf);   // accumulators of this tile complete
           }
-          umma_commit(empty0 + 8 * slot);   // frees the stage once these MMAs have read it
+          acc = 1u;
+          if (++slot == NS) { slot = 0; phase ^= 1u; }
         }
-        if (ok) umma_commit(acc_full0 + 8 * buf);   // accumulators of this tile complete
       }
     }
   } else if (warp >= 4) {
@@ -288,39 +404,55 @@ __global__ void __launch_bounds__(kGemmThreads, 1) tile_gemm_kernel(const __grid
     const int q = warp & 3, eg = (warp - 4) >> 2;
     constexpr int EG = kGemmEpiWarps / 4, CH = kGemmChunk;
     const int et = tid - 128;
+    const int rows_tile = kPair ? 2 * Rt : Rt;
+    const int nchunks = rows_tile / CH;
     griddep_wait();
     bool ok = true;
     int iter = 0;
     volatile int* last_flag = reinterpret_cast<volatile int*>(smem + 272);   // split-K: this CTA drew a tile's last ticket
-    for (int it = blockIdx.x; it < nitems_all && ok; it += gridDim.x, ++iter) {
+    // accumulator column of digit d of the tile's activation rows j0..j0+7
+    auto column = [&](int d, int j0) -> uint32_t {
+      if (!kPair) return uint32_t(d * Rt + j0);
+      const int h = j0 >= Rt ? 1 : 0, b = d * Rt + j0 - h * Rt;     // row b of CTA h's digit rows
+      return uint32_t(b < nb1 ? h * nb1 + b : kGemmAcc1Col + h * (nb - nb1) + b - nb1);
+    };
+    for (int it = first_item; it < nitems_all && ok; it += item_stride, ++iter) {
       const int tile = it / S;
       const GemmTile T = gemm_tile(P, tile);
       const GemmSeg& Sg = P.seg[T.seg];
-      const int n0 = T.n0, row0 = T.row0;
-      const bool two = P.mt == kGemmM && n0 + 128 < Sg.N;
+      const int n0 = T.n0 + rank * 128, row0 = T.row0;
       named_bar_sync(1, kGemmEpiWarps * 32);   // every epilogue warp is done with the previous tile's scalars
-      for (int i = et; i < Rt * 8; i += kGemmEpiWarps * 32) {
-        const int r = row0 + (i >> 3);
-        reinterpret_cast<float*>(scal)[i] = r < P.R ? __ldcg(reinterpret_cast<const float*>(Sg.scal + r) + (i & 7)) : 0.f;
+      for (int i = et; i < rows_tile * 4; i += kGemmEpiWarps * 32) {
+        const int r = row0 + (i >> 2);
+        scal[i] = r < P.R ? __ldcg(reinterpret_cast<const float*>(Sg.scal + r) + (i & 3)) : 0.f;
       }
       named_bar_sync(1, kGemmEpiWarps * 32);
       const int buf = dbuf ? (iter & 1) : 0, use = dbuf ? (iter >> 1) : iter;
       const uint32_t acc_empty = acc_empty0 + 8 * buf;
+      auto drained = [&]() {
+        tc_fence_before();
+        if (lane == 0) {
+          if (kPair) mbar_arrive_leader(acc_empty); else mbar_arrive(acc_empty);
+        }
+      };
       ok = __all_sync(0xffffffffu, mbar_wait_bounded(acc_full0 + 8 * buf, uint32_t(use & 1), abort_flag));
       if (!ok) {
         if (lane == 0 && P.status) atomicOr(P.status, B200RWKV_STATUS_WAIT_FULL);
         break;
       }
       tc_fence_after();
-      const int nchunks = Rt / CH, nitems = (two ? 2 : 1) * nchunks;
       // this warp's last item that really reads TMEM: after it the accumulators may be overwritten
       int last_item = -1;
-      for (int item = eg; item < nitems; item += EG)
-        if (row0 + (item % nchunks) * CH < P.R) last_item = item;
-      if (last_item < 0) {
-        tc_fence_before();
-        if (lane == 0) mbar_arrive(acc_empty);
-      }
+      for (int item = eg; item < nchunks; item += EG)
+        if (row0 + item * CH < P.R) last_item = item;
+      if (last_item < 0) drained();
+      auto load_digits = [&](int j0, int (&da)[CH], int (&db)[CH], int (&dc)[CH]) {
+        const uint32_t tbase = tmem + (uint32_t(q * 32) << 16) + uint32_t(buf * kGemmAcc1Col);
+        tmem_ld8(tbase + column(0, j0), da);
+        tmem_ld8(tbase + column(1, j0), db);
+        tmem_ld8(tbase + column(2, j0), dc);
+        tmem_ld_wait();
+      };
       // exact dot products of 8 rows of one output column from their three digit sums, as fp32
       auto recombine = [&](const int (&da)[CH], const int (&db)[CH], const int (&dc)[CH], float (&yf)[CH]) {
 #pragma unroll
@@ -328,8 +460,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1) tile_gemm_kernel(const __grid
           yf[j] = __ll2float_rn((long long)da[j] * 65536 + (long long)db[j] * 256 + (long long)dc[j]);
       };
       // affine terms + fused element-wise op for 8 rows of one output column
-      auto finish = [&](const float (&yf)[CH], int h, int j0) {
-        const int n = n0 + h * 128 + q * 32 + lane;
+      auto finish = [&](const float (&yf)[CH], int j0) {
+        const int n = n0 + q * 32 + lane;
         const bool nvalid = n < Sg.N;
         const int nc = nvalid ? n : Sg.N - 1;   // clamped: loads stay in bounds, the store is predicated
         const float rx = Sg.rx ? Sg.rx[nc] : 1.f, mx = Sg.mx ? Sg.mx[nc] : 0.f;
@@ -337,7 +469,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) tile_gemm_kernel(const __grid
         float yv[CH];
 #pragma unroll
         for (int j = 0; j < CH; ++j) {
-          const float4 sc = *reinterpret_cast<const float4*>(&scal[j0 + j]);   // sd, zp, sumxs, sumx
+          const float4 sc = reinterpret_cast<const float4*>(scal)[j0 + j];   // sd, zp, sumxs, sumx
           float y = __fmul_rn(yf[j], sc.x) + Sg.half * sc.z;
           y *= rx;               // rx = 1, mx = 0 when the matrix has no per-output terms: exact no-ops
           y += sc.y;
@@ -372,57 +504,37 @@ __global__ void __launch_bounds__(kGemmThreads, 1) tile_gemm_kernel(const __grid
           if (r <= rlast && nvalid) Sg.out[size_t(r) * Sg.ldo + n] = yv[j];
         }
       };
-      // split-K scratch of this tile: [column = digit*Rt + row][128 weight rows] (mt = 128 only)
+      // split-K scratch of this tile: [column = digit*Rt + row][128 weight rows] (single-CTA tiles only)
       int* sk = S > 1 ? P.sk_acc + size_t(tile) * (kDigits * Rt) * 128 + q * 32 + lane : nullptr;
       if (S == 1) {
-        // Two passes, so that the accumulators are free again as early as possible (a 256-row tile has no
-        // second buffer: the next tile's MMAs wait for this): first every item of this warp leaves TMEM and
-        // is recombined to one fp32 per output (40 registers at most), then the affine terms, the gate and
+        // Two passes, so that the accumulators are free again as early as possible (a wide tile has no second
+        // buffer: the next tile's MMAs wait for this): first every item of this warp leaves TMEM and is
+        // recombined to one fp32 per output (40 registers at most), then the affine terms, the gate and
         // residual loads and the stores run from registers under the next tile's MMAs.
         float yf[kGemmItemsPerWarp][CH];
 #pragma unroll
         for (int u = 0; u < kGemmItemsPerWarp; ++u) {
           const int item = eg + u * EG;
-          if (item < nitems) {
-            const int h = item / nchunks, j0 = (item - h * nchunks) * CH;
-            if (row0 + j0 < P.R) {   // warp-uniform
-              const uint32_t tbase = tmem + (uint32_t(q * 32) << 16) + uint32_t((h + buf) * kGemmAcc1Col + j0);
-              int da[CH], db[CH], dc[CH];
-              tmem_ld8(tbase, da);
-              tmem_ld8(tbase + uint32_t(Rt), db);
-              tmem_ld8(tbase + uint32_t(2 * Rt), dc);
-              tmem_ld_wait();
-              if (item == last_item) {
-                tc_fence_before();
-                if (lane == 0) mbar_arrive(acc_empty);
-              }
-              recombine(da, db, dc, yf[u]);
-            }
+          if (item < nchunks && row0 + item * CH < P.R) {   // warp-uniform
+            int da[CH], db[CH], dc[CH];
+            load_digits(item * CH, da, db, dc);
+            if (item == last_item) drained();
+            recombine(da, db, dc, yf[u]);
           }
         }
 #pragma unroll
         for (int u = 0; u < kGemmItemsPerWarp; ++u) {
           const int item = eg + u * EG;
-          if (item < nitems) {
-            const int h = item / nchunks, j0 = (item - h * nchunks) * CH;
-            if (row0 + j0 < P.R) finish(yf[u], h, j0);
-          }
+          if (item < nchunks && row0 + item * CH < P.R) finish(yf[u], item * CH);
         }
       } else {
 #pragma unroll 1
-        for (int item = eg; item < nitems; item += EG) {
-          const int h = item / nchunks, j0 = (item - h * nchunks) * CH;
+        for (int item = eg; item < nchunks; item += EG) {
+          const int j0 = item * CH;
           if (row0 + j0 >= P.R) continue;   // warp-uniform
-          const uint32_t tbase = tmem + (uint32_t(q * 32) << 16) + uint32_t((h + buf) * kGemmAcc1Col + j0);
           int da[CH], db[CH], dc[CH];
-          tmem_ld8(tbase, da);
-          tmem_ld8(tbase + uint32_t(Rt), db);
-          tmem_ld8(tbase + uint32_t(2 * Rt), dc);
-          tmem_ld_wait();
-          if (item == last_item) {   // the rest works from registers: let the next tile's MMAs start
-            tc_fence_before();
-            if (lane == 0) mbar_arrive(acc_empty);
-          }
+          load_digits(j0, da, db, dc);
+          if (item == last_item) drained();   // the rest works from registers: let the next tile's MMAs start
 #pragma unroll
           for (int j = 0; j < CH; ++j) {   // 32 lanes = 32 consecutive ints per atomic instruction
             atomicAdd(sk + size_t(j0 + j) * 128, da[j]);
@@ -430,8 +542,6 @@ __global__ void __launch_bounds__(kGemmThreads, 1) tile_gemm_kernel(const __grid
             atomicAdd(sk + size_t(2 * Rt + j0 + j) * 128, dc[j]);
           }
         }
-      }
-      if (S > 1) {
         __threadfence();                                   // this thread's additions are visible before the ticket
         named_bar_sync(1, kGemmEpiWarps * 32);
         if (et == 0) {
@@ -458,7 +568,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) tile_gemm_kernel(const __grid
             }
             float yf[CH];
             recombine(da, db, dc, yf);
-            finish(yf, 0, j0);
+            finish(yf, j0);
           }
           if (et == 0) P.sk_count[tile] = 0u;
         }
@@ -469,19 +579,21 @@ __global__ void __launch_bounds__(kGemmThreads, 1) tile_gemm_kernel(const __grid
   tc_fence_before();
   __syncthreads();
   // After an aborted wait copies may still be in flight into this CTA's shared memory: give each
-  // issued copy a bounded chance to land before the CTA retires.
-  if (tid == 0 && *abort_flag) {
+  // issued copy a bounded chance to land before the CTA retires.  (The odd CTA of a pair has its bytes
+  // counted on the even CTA's barriers; neither retires before the cluster barrier below.)
+  if (tid == 0 && rank == 0 && *abort_flag) {
     const int issued = *issued_ptr;
     const unsigned long long t0 = globaltimer_ns();
-    for (int i = issued > kGemmStages ? issued - kGemmStages : 0; i < issued; ++i) {
-      const uint32_t bar = full0 + 8 * (i % kGemmStages), parity = uint32_t(i / kGemmStages) & 1u;
+    for (int i = issued > NS ? issued - NS : 0; i < issued; ++i) {
+      const uint32_t bar = full0 + 8 * (i % NS), parity = uint32_t(i / NS) & 1u;
       while (!mbar_try_wait(bar, parity) && globaltimer_ns() - t0 < kWaitLimitNs / 10) {
       }
     }
   }
+  if (kPair) cluster_sync();             // nothing of the pair's work touches either CTA any more
   if (warp == 2) {
     tc_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kGemmTmemCols) : "memory");
+    tmem_dealloc<kPair>(tmem);
   }
 }
 
@@ -586,7 +698,7 @@ __device__ __forceinline__ float4 ln_apply(float4 x, float mean, float rstd, flo
 template <int NT, int NV, bool MAX0>
 __device__ __forceinline__ void span_reduce(float (&v)[NV], float* red, int& phase) {
   constexpr int NW = NT / 32;
-  static_assert(NV <= 4 && (NW == 8 || NW == 16), "one float4 slot per warp, 8 or 16 warps");
+  static_assert(NV <= 4 && (NW == 8 || NW == 16 || NW == 32), "one float4 slot per warp; a power of two of warps");
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
   for (int k = 0; k < NV; ++k) v[k] = (MAX0 && k == 0) ? warp_max(v[k]) : warp_sum(v[k]);
@@ -873,14 +985,31 @@ __device__ __forceinline__ void rows_prep_long(const RowsPrepParams& P, float* r
 // row needs (fewer registers, more resident CTAs).  256 threads while a row fits, else 512.
 constexpr int kRowsPrepGroupsLn = 4, kRowsPrepGroupsPlain = 8;
 constexpr int rows_prep_min_ctas(int NT, int mode, int G) {
-  return mode == ROWS_LN ? (NT == 256 ? (G <= 2 ? 5 : G == 3 ? 4 : 3) : (G <= 3 ? 2 : 1))
+  return NT == 1024 ? 2 : mode == ROWS_LN ? (NT == 256 ? (G <= 2 ? 5 : G == 3 ? 4 : 3) : (G <= 3 ? 2 : 1))
                          : (NT == 256 ? (G <= 4 ? 5 : 4) : 2);
+}
+
+// Parameter vectors of the launch -> L2, by the CTAs of the first rows (see prefetch_l2_floats).
+template <int NT>
+__device__ __forceinline__ void rows_prep_prefetch(const RowsPrepParams& P) {
+  if (blockIdx.y != 0) return;
+  const int s0 = P.segs_per_cta == 1 ? int(blockIdx.x) : 0, s1 = P.segs_per_cta == 1 ? s0 + 1 : P.nseg;
+  if (s0 == 0) {
+    prefetch_l2_floats(P.ln_w, P.K, threadIdx.x, NT);
+    prefetch_l2_floats(P.ln_b, P.K, threadIdx.x, NT);
+  }
+  for (int s = s0; s < s1; ++s) {
+    prefetch_l2_floats(P.seg[s].mix, P.K, threadIdx.x, NT);
+    prefetch_l2_floats(P.seg[s].ry, P.K, threadIdx.x, NT);
+    prefetch_l2_floats(P.seg[s].my, P.K, threadIdx.x, NT);
+  }
 }
 
 template <int NT, int MODE, int G>
 __global__ void __launch_bounds__(NT, rows_prep_min_ctas(NT, MODE, G)) rows_prep_kernel(const __grid_constant__ RowsPrepParams P) {
   extern __shared__ __align__(128) unsigned char prep_smem[];
   griddep_launch_dependents();
+  rows_prep_prefetch<NT>(P);
   griddep_wait();
   rows_prep_span<NT, G, MODE == ROWS_LN>(P, reinterpret_cast<float*>(prep_smem));
 }
@@ -889,6 +1018,7 @@ __global__ void __launch_bounds__(NT, rows_prep_min_ctas(NT, MODE, G)) rows_prep
 __global__ void __launch_bounds__(512, 2) rows_prep_long_kernel(const __grid_constant__ RowsPrepParams P) {
   extern __shared__ __align__(128) unsigned char prep_smem[];
   griddep_launch_dependents();
+  rows_prep_prefetch<512>(P);
   griddep_wait();
   rows_prep_long<512>(P, reinterpret_cast<float*>(prep_smem), reinterpret_cast<float4*>(prep_smem + kPrepRedBytes));
 }
