@@ -641,7 +641,7 @@ static cudaError_t launch_tile_gemm_as(GemmParams& P, const b200rwkv_matrix* con
   const int weight_rows = pair ? 2 * kGemmM : kGemmM, rows_tile = pair ? 2 * Rt : Rt;
   P.dbuf = kDigits * rows_tile <= kGemmAcc1Col ? 1 : 0;
   const int chunk = (kGemmM + kDigits * Rt) * 128, nk = P.K / 128 / ksplit;
-  P.kc = kc > 0 ? kc : gemm_chunks_per_stage(chunk, nk);
+  P.kc = kc > 0 ? kc : gemm_chunks_per_stage(chunk, nk, pair);
   P.stage_bytes = P.kc * chunk;
   P.stages = std::min(kGemmRingBytes / P.stage_bytes, kGemmMaxStages);
   for (int s = 0; s < P.nseg; ++s) {
@@ -672,10 +672,10 @@ static cudaError_t launch_tile_gemm_as(GemmParams& P, const b200rwkv_matrix* con
 // besides).  The step times (128 bytes of K, us) are measured on launches of one round (7B ffn value,
 // K = 16384, 16 to 320 rows); they are shared-memory traffic (operands in by TMA, out to the tensor
 // core), which is why a pair, whose CTAs each hold half of the digit rows, needs less per row.  A tile
-// whose accumulator has no second buffer waits about 3 us for its epilogue; so does a K slice for its
+// whose accumulator has no second buffer waits 3.6 us for its epilogue; a K slice pays 3 us for its
 // atomics and ticket.
 static void gemm_pick_tile(const GemmParams& P, int* pair, int* Rt, int* ksplit) {
-  static const double step_single[5] = {0.19, 0.24, 0.335, 0.345, 0.37}, step_pair[5] = {0.22, 0.325, 0.40, 0.455, 0.565};   // Rt = 16, 32, .. 80
+  static const double step_single[5] = {0.16, 0.215, 0.26, 0.32, 0.345}, step_pair[5] = {0.18, 0.25, 0.40, 0.45, 0.555};   // Rt = 16, 32, .. 80
   const long long sms = device_sms() > 1 ? device_sms() : 2;
   const int nk = P.K / 128;
   double best = 0.0;
@@ -694,7 +694,7 @@ static void gemm_pick_tile(const GemmParams& P, int* pair, int* Rt, int* ksplit)
           continue;
         const long long units = pr ? sms / 2 : sms;
         const double rounds = double((tiles * ks + units - 1) / units);
-        const double cost = rounds * (double(nk / ks) * (pr ? step_pair[i] : step_single[i]) + (ks > 1 || !dbuf ? 3.0 : 0.8));
+        const double cost = rounds * (double(nk / ks) * (pr ? step_pair[i] : step_single[i]) + (ks > 1 ? 3.0 : dbuf ? 1.2 : 3.6));
         if (best == 0.0 || cost < best) { best = cost; *pair = pr; *Rt = rt; *ksplit = ks; }
       }
     }
@@ -1080,61 +1080,84 @@ static DenseRowsWorkspace dense_carve_rows(const b200rwkv_dense_model* m, int B,
   return w;
 }
 
-// Picks the tile, encodes the tensor maps and launches.  w[s]: [N_s][K] of the 16-bit
-// type; x[s]: [rows_alloc][K] of the same type.
-static cudaError_t launch_dense_gemm(DGemmParams& P, const void* const* w, const unsigned short* const* x, int K, int rows_alloc,
-                                     cudaStream_t stream, const char** why) {
+// Encodes the tensor maps for one tile shape and launches.  w[s]: [N_s][K] of the 16-bit type; x[s]:
+// [rows_alloc][K] of the same type.
+static cudaError_t launch_dense_gemm_as(DGemmParams& P, const void* const* w, const unsigned short* const* x, int K, int rows_alloc,
+                                        bool pair, int Rt, int ksplit, int kc, cudaStream_t stream, const char** why) {
   static bool configured[64];
   *why = "dense_tile_gemm launch failed";
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
   if (dev >= 0 && dev < 64 && !configured[dev]) {
-    e = cudaFuncSetAttribute(dense_tile_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kDgSmem);
+    e = cudaFuncSetAttribute(dense_tile_gemm_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kDgSmem);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(dense_tile_gemm_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kDgSmem);
     if (e != cudaSuccess) return e;
     configured[dev] = true;
   }
-  const int sms = device_sms();
   P.ksteps = K * 2 / 128;
-  // Tile: rounds of tiles per CTA x (operand bytes of a tile + a fixed cost per tile), over both tile
-  // widths and every height that splits the rows evenly.
-  double best = 0.0;
-  for (int mt = 128; mt <= 256; mt += 128) {
-    for (int rt_rows = 1; rt_rows <= (P.R + 15) / 16; ++rt_rows) {
-      const int rt = gemm_padded_rows((P.R + rt_rows - 1) / rt_rows);
-      if (rt > kDgRowsMax) continue;
-      const int row_tiles = (P.R + rt - 1) / rt;
-      if (row_tiles != rt_rows) continue;
-      long long tiles = 0;
-      for (int s = 0; s < P.nseg; ++s) tiles += (long long)row_tiles * ((P.seg[s].N + mt - 1) / mt);
-      for (int ks = 1; ks <= 8; ks *= 2) {     // K slices: only where few tiles would leave most SMs idle
-        if (ks > 1 && (!P.sk_part || mt != 128 || tiles * ks > kDgSplitMaxItems || tiles * ks * rt > kDgSplitMaxCells ||
-                       P.ksteps % ks != 0 || P.ksteps / ks < 4))
-          continue;
-        const double rounds = double((tiles * ks + sms - 1) / sms);
-        const double reduce = ks > 1 ? 2.0 * rt * 128 * 4 + 64.0 * 1024 : 0.0;   // partial sums out and back, ticket
-        const double cost = rounds * (double(P.ksteps / ks) * 128.0 * (mt + rt) + 48.0 * 1024 + reduce);
-        if (best == 0.0 || cost < best) { best = cost; P.mt = mt; P.Rt = rt; P.ksplit = ks; }
-      }
-    }
-  }
-  if (best == 0.0) { *why = "no tile fits"; return cudaErrorInvalidValue; }
-  P.row_tiles = (P.R + P.Rt - 1) / P.Rt;
-  P.stage_bytes = (P.mt + P.Rt) * 128;
-  P.stages = kDgRingBytes / P.stage_bytes < kDgMaxStages ? kDgRingBytes / P.stage_bytes : kDgMaxStages;
+  P.pair = pair ? 1 : 0; P.Rt = Rt; P.ksplit = ksplit;
+  const int weight_rows = pair ? 256 : 128, rows_tile = pair ? 2 * Rt : Rt, chunk = (128 + Rt) * 128;
+  P.kc = kc > 0 ? kc : gemm_chunks_per_stage(chunk, P.ksteps / ksplit, pair);
+  P.stage_bytes = P.kc * chunk;
+  P.stages = std::min(kDgRingBytes / P.stage_bytes, kDgMaxStages);
+  P.row_tiles = (P.R + rows_tile - 1) / rows_tile;
   P.ntiles = 0;
   for (int s = 0; s < P.nseg; ++s) {
-    if (!encode_byte_map(&P.seg[s].wmap, w[s], (unsigned long long)P.seg[s].N, K * 2, P.mt, 1) ||
-        !encode_byte_map(&P.seg[s].xmap, x[s], (unsigned long long)rows_alloc, K * 2, P.Rt, 1)) {
+    if (!encode_byte_map(&P.seg[s].wmap, w[s], (unsigned long long)P.seg[s].N, K * 2, 128, P.kc) ||
+        !encode_byte_map(&P.seg[s].xmap, x[s], (unsigned long long)rows_alloc, K * 2, Rt, P.kc)) {
       *why = "cuTensorMapEncodeTiled failed";
       return cudaErrorInvalidValue;
     }
-    P.tiles_seg[s] = P.row_tiles * ((P.seg[s].N + P.mt - 1) / P.mt);
+    P.tiles_seg[s] = P.row_tiles * ((P.seg[s].N + weight_rows - 1) / weight_rows);
     P.ntiles += P.tiles_seg[s];
   }
-  const int items = P.ntiles * P.ksplit;
-  const dim3 grid(items < sms ? items : sms);
-  return launch_chained(dense_tile_gemm_kernel, grid, dim3(kGemmThreads), size_t(kDgSmem), stream, P);
+  const int items = P.ntiles * P.ksplit, sms = device_sms();
+  if (pair) {
+    const int pairs = items < sms / 2 ? items : sms / 2;
+    return launch_clustered(2, dense_tile_gemm_kernel<true>, dim3(2 * pairs), dim3(kGemmThreads), size_t(kDgSmem), stream, P);
+  }
+  return launch_chained(dense_tile_gemm_kernel<false>, dim3(items < sms ? items : sms), dim3(kGemmThreads), size_t(kDgSmem), stream, P);
+}
+
+// Time of one K step (64 elements) of a tile, us: straight lines through launches of one round (7B ffn
+// value, K = 16384, 16 to 240 rows), one for each number of chunks per stage.  Tiles are chosen like
+// gemm_pick_tile's, by rounds x (K steps x step time + what a tile or slice costs besides).
+static double dense_gemm_step_us(bool pair, int Rt) {
+  const bool two = gemm_chunks_per_stage((128 + Rt) * 128, 2, pair) == 2;
+  return pair ? (two ? 0.125 + 0.0012 * Rt : 0.16 + 0.00105 * Rt) : (two ? 0.14 + 0.00085 * Rt : 0.15 + 0.0009 * Rt);
+}
+
+static bool dense_gemm_pick_tile(const DGemmParams& P, int ksteps, int* pair, int* Rt, int* ksplit) {
+  const int sms = device_sms() > 1 ? device_sms() : 2;
+  double best = 0.0;
+  for (int pr = 0; pr <= 1; ++pr) {
+    const int unit = pr ? 32 : 16, most = pr ? 2 * kDgRowsPair : kDgRowsSingle;
+    for (int rt_rows = 1; rt_rows <= (P.R + unit - 1) / unit; ++rt_rows) {
+      const int rows = ((P.R + rt_rows - 1) / rt_rows + unit - 1) / unit * unit;
+      if (rows > most || (P.R + rows - 1) / rows != rt_rows) continue;
+      long long tiles = 0;
+      for (int s = 0; s < P.nseg; ++s) tiles += (long long)rt_rows * ((P.seg[s].N + (pr ? 255 : 127)) / (pr ? 256 : 128));
+      for (int ks = 1; ks <= 8; ks *= 2) {     // K slices: only where few tiles would leave most SMs idle
+        if (ks > 1 && (!P.sk_part || pr || tiles * ks > kDgSplitMaxItems || tiles * ks * rows > kDgSplitMaxCells ||
+                       ksteps % ks != 0 || ksteps / ks < 4))
+          continue;
+        const double step = dense_gemm_step_us(pr != 0, pr ? rows / 2 : rows);
+        const double rounds = double(pr ? (tiles + sms / 2 - 1) / (sms / 2) : (tiles * ks + sms - 1) / sms);
+        const double cost = rounds * (double(ksteps / ks) * step + (ks > 1 ? 3.0 : 1.0));
+        if (best == 0.0 || cost < best) { best = cost; *pair = pr; *Rt = pr ? rows / 2 : rows; *ksplit = ks; }
+      }
+    }
+  }
+  return best != 0.0;
+}
+
+// Picks the tile and launches (see launch_dense_gemm_as).
+static cudaError_t launch_dense_gemm(DGemmParams& P, const void* const* w, const unsigned short* const* x, int K, int rows_alloc,
+                                     cudaStream_t stream, const char** why) {
+  int pair = 0, Rt = 16, ksplit = 1;
+  if (!dense_gemm_pick_tile(P, K * 2 / 128, &pair, &Rt, &ksplit)) { *why = "no tile fits"; return cudaErrorInvalidValue; }
+  return launch_dense_gemm_as(P, w, x, K, rows_alloc, pair != 0, Rt, ksplit, 0, stream, why);
 }
 
 static void fill_dgemm_seg(DGemmSeg& s, int N, void* out, long long ldo, int act, int out_t) {

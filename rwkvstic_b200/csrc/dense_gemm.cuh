@@ -5,14 +5,15 @@
 //
 //   out[r][n] = epilogue( round_T( sum_k x_T[r][k] * W[n][k] ) )        fp32 accumulation
 //
-//   A = mt weight rows     x 128 bytes of K (64 elements; one TMA box of W[N][K], 128-byte swizzle; mt = 128 or 256)
-//   B = Rt activation rows x 128 bytes of K (one TMA box of the rows already rounded to T; Rt = 16..240)
-//   D = 128 lanes x Rt fp32 columns per 128 weight rows in tensor memory; a 256-row tile keeps its
-//       second accumulator at column 256, with 128-row tiles columns 0 and 256 are two buffers.
+//   A = 128 weight rows    x 128 bytes of K (64 elements; a TMA box of W[N][K], 128-byte swizzle)
+//   B = Rt activation rows x 128 bytes of K (a TMA box of the rows already rounded to T; Rt = 16..240)
+//   D = 128 lanes x activation rows fp32 columns in tensor memory, two buffers (columns 0 and 256): the
+//       epilogue of a tile runs under the MMAs of the next.
 //
-// Same skeleton as tile_gemm.cuh (persistent CTAs, a three-stage operand ring that runs on across
-// tiles, warp 0 = TMA producer, warp 1 = MMA issuer with tcgen05.mma kind::f16, warps 4..19 =
-// epilogue through tcgen05.ld); no digit planes, no per-row scalars.  With few rows and therefore few
+// Same skeleton and the same two forms as tile_gemm.cuh: a CTA on 128 weight rows x Rt activation rows, or
+// a pair of CTAs (tcgen05.mma.cta_group::2) on 256 x 2*Rt, up to 256 x 256.  Persistent CTAs, an operand
+// ring that runs on across tiles, warp 0 = TMA producer, warp 1 = MMA issuer (kind::f16), warps 4..19 =
+// epilogue through tcgen05.ld; no digit planes, no per-row scalars.  With few rows and therefore few
 // tiles K is cut into slices (work item = tile x slice): a slice parks its fp32 partial sums in a scratch
 // buffer and draws a ticket; the CTA that draws a tile's last ticket adds the slices IN SLICE ORDER (so
 // the result does not depend on which CTA finished when) and runs the epilogue.  Nobody waits for anybody.
@@ -25,10 +26,8 @@
 
 namespace b200 {
 
-constexpr int kDgM = 256;
-constexpr int kDgRowsMax = 240;                                  // activation rows per tile: 30 KB of a stage
-constexpr int kDgStageBytes = (kDgM + kDgRowsMax) * 128;    // 62 KB
-constexpr int kDgRingBytes = 3 * kDgStageBytes;          // 186 KB: three stages of the largest tile, up to eight of a small one
+constexpr int kDgRowsSingle = 240, kDgRowsPair = 128;            // activation rows a CTA holds of a tile, at most
+constexpr int kDgRingBytes = 186 * 1024;
 constexpr int kDgMaxStages = 8;                                  // barriers: full 0..7, empty 8..15
 constexpr int kDgSmem = kGemmOffRing + kDgRingBytes;
 constexpr int kDgSplitMaxItems = 640;                            // tiles x slices of a split launch (its tickets)
@@ -37,8 +36,8 @@ constexpr long long kDgSplitMaxCells = 640ll * 64;               // tiles x slic
 constexpr size_t kDgSplitBytes = size_t(kDgSplitMaxCells) * 128 * 4;   // 21 MB of partial sums
 
 struct DGemmSeg {
-  CUtensorMap wmap;     // W as bytes [K*2/128][N][128 B], box [1][mt][128], 128-byte swizzle
-  CUtensorMap xmap;     // rows as bytes [K*2/128][Rpad][128 B], box [1][Rt][128], 128-byte swizzle
+  CUtensorMap wmap;     // W as bytes [K*2/128][N][128 B], box [kc][128][128], 128-byte swizzle
+  CUtensorMap xmap;     // rows as bytes [K*2/128][Rpad][128 B], box [kc][Rt][128], 128-byte swizzle
   void* out;            // [R][ldo] of float, or of T when out_t is set
   const float* res;     // [R][ldres] added last, or null
   const float* gate;    // [R][ldgate] multiplies the product first, or null
@@ -49,13 +48,15 @@ struct DGemmSeg {
 struct DGemmParams {
   DGemmSeg seg[kMaxSeg];
   int nseg, ksteps, R;  // ksteps = K * 2 / 128
-  int Rt, mt, row_tiles;
+  int pair;             // tiles of a CTA pair: 256 weight rows x 2*Rt activation rows; else 128 x Rt
+  int Rt, row_tiles;
   int tiles_seg[kMaxSeg];
   int ntiles;
   int is_bf16;
+  int kc;               // K steps of 128 bytes per stage, 1 or 2
   int stages;           // ring depth: as many stages of stage_bytes as fit the ring, at most 8
-  int stage_bytes;      // mt * 128 (weights) + Rt * 128 (rows), a multiple of 1024
-  int ksplit;           // K slices per tile (1: none; > 1 only with 128-row tiles; divides ksteps)
+  int stage_bytes;      // kc * (128 + Rt) * 128, a multiple of 1024
+  int ksplit;           // K slices per tile (1: none; > 1 only with single-CTA tiles; divides ksteps)
   float* sk_part;       // [ntiles][ksplit][Rt][128] partial sums of the slices
   unsigned* sk_count;   // [ntiles] tickets, zero between launches
   int* status;
@@ -67,12 +68,20 @@ __host__ __device__ constexpr uint32_t umma_idesc_f16(int M, int N, int is_bf16)
          (uint32_t(M >> 4) << 24);
 }
 
+template <bool kPair>
 __device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
-      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
+  if constexpr (kPair)
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
+        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        : "memory");
+  else
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
+        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        : "memory");
 }
 
 __device__ __forceinline__ float round16(float v, int is_bf16) {
@@ -87,22 +96,26 @@ __device__ __forceinline__ DGemmTile dgemm_tile(const DGemmParams& P, int t) {
   int s = 0;
   while (s < P.nseg - 1 && t >= P.tiles_seg[s]) { t -= P.tiles_seg[s]; ++s; }
   const int wt = t / P.row_tiles;                       // tiles that share a weight tile are consecutive
-  return {s, wt * P.mt, (t - wt * P.row_tiles) * P.Rt};
+  return {s, wt * (P.pair ? 256 : 128), (t - wt * P.row_tiles) * (P.pair ? 2 * P.Rt : P.Rt)};
 }
 
+// kPair: two CTAs of a cluster work on one tile with tcgen05.mma.cta_group::2 (see tile_gemm.cuh).
+template <bool kPair>
 __global__ void __launch_bounds__(kGemmThreads, 1) dense_tile_gemm_kernel(const __grid_constant__ DGemmParams P) {
   extern __shared__ __align__(1024) unsigned char smem[];
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = warp_index(), lane = tid & 31;
   const int Rt = P.Rt, S = P.ksplit;
   const int nk = P.ksteps / S;            // K steps of one work item
   const int nitems_all = P.ntiles * S;
-  const int NS = P.stages;
-  const uint32_t a_bytes = uint32_t(P.mt) * 128u, b_bytes = uint32_t(Rt) * 128u;
+  const int NS = P.stages, KC = P.kc;
+  const int rank = kPair ? int(cluster_ctarank()) : 0;                    // which half of the tile this CTA holds
+  const int first_item = kPair ? int(blockIdx.x >> 1) : int(blockIdx.x), item_stride = kPair ? int(gridDim.x >> 1) : int(gridDim.x);
+  const uint32_t a_chunk = 128u * 128u, b_chunk = uint32_t(Rt) * 128u;
+  const uint32_t a_bytes = uint32_t(KC) * a_chunk;      // a stage: KC weight chunks, then KC row chunks
 
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem);
   const uint32_t full0 = smem_u32(bars), empty0 = smem_u32(bars + 8);
   const uint32_t acc_full0 = smem_u32(bars + 16), acc_empty0 = smem_u32(bars + 18);
-  const bool dbuf = P.mt != kDgM;
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + 256);
   volatile int* issued_ptr = reinterpret_cast<volatile int*>(smem + 260);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + 264);
@@ -110,97 +123,95 @@ __global__ void __launch_bounds__(kGemmThreads, 1) dense_tile_gemm_kernel(const 
 
   if (tid == 0) {
     for (int i = 0; i < kDgMaxStages; ++i) { mbar_init(full0 + 8 * i, 1); mbar_init(empty0 + 8 * i, 1); }
-    for (int i = 0; i < 2; ++i) { mbar_init(acc_full0 + 8 * i, 1); mbar_init(acc_empty0 + 8 * i, kGemmEpiWarps); }
+    for (int i = 0; i < 2; ++i) { mbar_init(acc_full0 + 8 * i, 1); mbar_init(acc_empty0 + 8 * i, (kPair ? 2 : 1) * kGemmEpiWarps); }
     *abort_flag = 0;
     *issued_ptr = 0;
     fence_mbar_init();
   }
-  if (warp == 2) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(kGemmTmemCols) : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-  }
+  if (warp == 2) tmem_alloc<kPair>(smem_u32(tmem_slot));
   tc_fence_before();
   __syncthreads();
+  if (kPair) cluster_sync();             // the partner's barriers exist before anything arrives on them
   tc_fence_after();
-  const uint32_t tmem = *tmem_slot;
+  const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
   griddep_launch_dependents();
 
   if (warp == 0) {
     // ---------------------------------------------------------------- TMA producer
-    if (lane == 0) {
-      int issued = 0;
-      bool ok = true;
-      // Weights are constants: the first ring of them is requested before the launch dependency resolves.
-      int early = 0;
-      for (int it = blockIdx.x; it < nitems_all && early < NS; it += gridDim.x) {
-        const DGemmTile T = dgemm_tile(P, it / S);
-        for (int kc = 0; kc < nk && early < NS; ++kc, ++early) {
-          mbar_arrive_expect_tx(full0 + 8 * early, a_bytes + b_bytes);
-          tma_load_3d(smem_u32(ring + size_t(early) * P.stage_bytes), &P.seg[T.seg].wmap, 0, T.n0, (it % S) * nk + kc, full0 + 8 * early);
-        }
+    const uint32_t ring0 = smem_u32(ring), stage_bytes = uint32_t(P.stage_bytes);
+    const uint32_t full_at = kPair ? leader_addr(full0) : full0;
+    const uint32_t tx_bytes = kPair ? 2u * stage_bytes : stage_bytes;
+    struct Cursor { int it, k, left; DGemmTile T; };      // work item, K step of the copy, K steps left of the item
+    auto start = [&](Cursor& c) {
+      if (c.it < nitems_all) { c.T = dgemm_tile(P, c.it / S); c.k = S == 1 ? 0 : (c.it % S) * nk; c.left = nk; }
+    };
+    auto next = [&](Cursor& c) {
+      c.k += KC;
+      if ((c.left -= KC) <= 0) { c.it += item_stride; start(c); }
+    };
+    Cursor ld;
+    ld.it = first_item;
+    start(ld);
+    // Weights are constants: the first ring of them is requested before the launch dependency resolves.
+    int early = 0;
+    for (; early < NS && ld.it < nitems_all; ++early, next(ld)) {
+      if (elect_one()) {
+        if (rank == 0) mbar_arrive_expect_tx(full0 + 8 * early, tx_bytes);
+        tma_operand_3d<kPair>(ring0 + uint32_t(early) * stage_bytes, &P.seg[ld.T.seg].wmap, 0, ld.T.n0 + rank * 128, ld.k, full_at + 8 * early);
       }
-      *issued_ptr = early;
-      griddep_wait();   // the activation rows come from the kernel in front of this launch
-      for (int it = blockIdx.x; it < nitems_all && ok; it += gridDim.x) {
-        const DGemmTile T = dgemm_tile(P, it / S);
-        const DGemmSeg& Sg = P.seg[T.seg];
-        const int kbase = (it % S) * nk;
-        for (int kc = 0; kc < nk; ++kc, ++issued) {
-          const int slot = issued % NS;
-          const uint32_t bar = full0 + 8 * slot;
-          const uint32_t dst = smem_u32(ring + size_t(slot) * P.stage_bytes);
-          if (issued >= early) {
-            const uint32_t phase = uint32_t(issued / NS) & 1u;
-            if (!mbar_wait_bounded(empty0 + 8 * slot, phase ^ 1u, abort_flag)) {
-              if (P.status) atomicOr(P.status, B200RWKV_STATUS_WAIT_EMPTY);
-              ok = false;
-              break;
-            }
-            mbar_arrive_expect_tx(bar, a_bytes + b_bytes);
-            tma_load_3d(dst, &Sg.wmap, 0, T.n0, kbase + kc, bar);                    // rows past N are zero-filled
-          }
-          tma_load_3d(dst + a_bytes, &Sg.xmap, 0, T.row0, kbase + kc, bar);    // rows past the buffer too
-        }
-      }
-      *issued_ptr = issued;
     }
+    *issued_ptr = early;
+    griddep_wait();   // the activation rows come from the kernel in front of this launch
+    int issued = 0, slot = 0;
+    uint32_t phase = 0;
+    ld.it = first_item;
+    for (start(ld); ld.it < nitems_all; next(ld)) {
+      const DGemmSeg& Sg = P.seg[ld.T.seg];
+      const uint32_t bar = full_at + 8 * slot, dst = ring0 + uint32_t(slot) * stage_bytes;
+      if (issued >= early) {
+        if (!warp_wait(empty0 + 8 * slot, phase ^ 1u, abort_flag, P.status, B200RWKV_STATUS_WAIT_EMPTY)) break;
+        if (elect_one()) {
+          if (rank == 0) mbar_arrive_expect_tx(full0 + 8 * slot, tx_bytes);
+          tma_operand_3d<kPair>(dst, &Sg.wmap, 0, ld.T.n0 + rank * 128, ld.k, bar);   // rows past N are zero-filled
+        }
+      }
+      if (elect_one()) tma_operand_3d<kPair>(dst + a_bytes, &Sg.xmap, 0, ld.T.row0 + rank * Rt, ld.k, bar);   // rows past the buffer too
+      ++issued;
+      if (++slot == NS) { slot = 0; phase ^= 1u; }
+    }
+    *issued_ptr = issued;
   } else if (warp == 1) {
-    // ---------------------------------------------------------------- MMA issuer
-    if (lane == 0) {
-      const uint32_t idesc = umma_idesc_f16(128, Rt, P.is_bf16);
+    // ---------------------------------------------------------------- MMA issuer (the even CTA's, for both)
+    if (rank == 0) {
+      const uint32_t idesc = umma_idesc_f16(kPair ? 256 : 128, kPair ? 2 * Rt : Rt, P.is_bf16);
+      const uint32_t ring0 = smem_u32(ring), stage_bytes = uint32_t(P.stage_bytes);
       bool ok = true;
-      int step = 0, iter = 0;
-      for (int it = blockIdx.x; it < nitems_all && ok; it += gridDim.x, ++iter) {
-        const DGemmTile T = dgemm_tile(P, it / S);
-        const bool two = P.mt == kDgM && T.n0 + 128 < P.seg[T.seg].N;
-        const int buf = dbuf ? (iter & 1) : 0, use = dbuf ? (iter >> 1) : iter;
+      int iter = 0, slot = 0;
+      uint32_t phase = 0;
+      for (int it = first_item; it < nitems_all && ok; it += item_stride, ++iter) {
+        const int buf = iter & 1, use = iter >> 1;
         const uint32_t tacc = tmem + uint32_t(buf * kGemmAcc1Col);
-        if (!mbar_wait_bounded(acc_empty0 + 8 * buf, uint32_t(use & 1) ^ 1u, abort_flag)) {
-          if (P.status) atomicOr(P.status, B200RWKV_STATUS_WAIT_EMPTY);
-          ok = false;
-          break;
-        }
-        tc_fence_after();
-        for (int kc = 0; kc < nk; ++kc, ++step) {
-          const int slot = step % NS;
-          const uint32_t phase = uint32_t(step / NS) & 1u;
-          if (!mbar_wait_bounded(full0 + 8 * slot, phase, abort_flag)) {
-            if (P.status) atomicOr(P.status, B200RWKV_STATUS_WAIT_FULL);
-            ok = false;
-            break;
-          }
-          tc_fence_after();
-          const uint32_t a = smem_u32(ring + size_t(slot) * P.stage_bytes);
-          const uint64_t ad0 = umma_desc(a), ad1 = umma_desc(a + 128 * 128), bd = umma_desc(a + a_bytes);
+        if (!warp_wait(acc_empty0 + 8 * buf, uint32_t(use & 1) ^ 1u, abort_flag, P.status, B200RWKV_STATUS_WAIT_EMPTY)) break;
+        uint32_t acc = 0u;    // the first MMA of a tile overwrites the accumulator
+        for (int k0 = 0; k0 < nk; k0 += KC) {
+          if (!warp_wait(full0 + 8 * slot, phase, abort_flag, P.status, B200RWKV_STATUS_WAIT_FULL)) { ok = false; break; }
+          if (elect_one()) {
+            tc_fence_after();
+            const uint32_t a = ring0 + uint32_t(slot) * stage_bytes;
+            const uint64_t ad = umma_desc(a), bd = umma_desc(a + a_bytes);
+            auto chunk = [&](uint64_t a64, uint64_t b64, uint32_t first) {    // straight-line issue, see tile_gemm.cuh
 #pragma unroll
-          for (int k = 0; k < 4; ++k) {   // 16 elements = 32 bytes of K per instruction: +2 in the descriptors' 16-byte units
-            const uint32_t acc = (kc | k) != 0 ? 1u : 0u;
-            umma_f16(tacc, ad0 + uint64_t(2 * k), bd + uint64_t(2 * k), idesc, acc);
-            if (two) umma_f16(tmem + kGemmAcc1Col, ad1 + uint64_t(2 * k), bd + uint64_t(2 * k), idesc, acc);
+              for (int k = 0; k < 4; ++k)   // 16 elements = 32 bytes of K per instruction: +2 in the descriptors' 16-byte units
+                umma_f16<kPair>(tacc, a64 + uint64_t(2 * k), b64 + uint64_t(2 * k), idesc, k == 0 ? first : 1u);
+            };
+            chunk(ad, bd, acc);
+            if (KC > 1 && nk - k0 > 1) chunk(ad + uint64_t(a_chunk >> 4), bd + uint64_t(b_chunk >> 4), 1u);
+            umma_commit<kPair>(empty0 + 8 * slot);
+            if (k0 + KC >= nk) umma_commit<kPair>(acc_full0 + 8 * buf);
           }
-          umma_commit<false>(empty0 + 8 * slot);
+          acc = 1u;
+          if (++slot == NS) { slot = 0; phase ^= 1u; }
         }
-        if (ok) umma_commit<false>(acc_full0 + 8 * buf);
       }
     }
   } else if (warp >= 4) {
@@ -208,36 +219,38 @@ __global__ void __launch_bounds__(kGemmThreads, 1) dense_tile_gemm_kernel(const 
     const int q = warp & 3, eg = (warp - 4) >> 2;
     constexpr int EG = kGemmEpiWarps / 4, CH = kGemmChunk;
     const int et = tid - 128;
+    const int rows_tile = kPair ? 2 * Rt : Rt, nchunks = rows_tile / CH;   // TMEM column = row of the tile
     volatile int* last_flag = reinterpret_cast<volatile int*>(smem + 272);   // K split: this CTA drew a tile's last ticket
     griddep_wait();
     bool ok = true;
     int iter = 0;
-    for (int it = blockIdx.x; it < nitems_all && ok; it += gridDim.x, ++iter) {
+    for (int it = first_item; it < nitems_all && ok; it += item_stride, ++iter) {
       const int tile = it / S, slice = it - tile * S;
       const DGemmTile T = dgemm_tile(P, tile);
       const DGemmSeg& Sg = P.seg[T.seg];
-      const int n0 = T.n0, row0 = T.row0;
-      const bool two = P.mt == kDgM && n0 + 128 < Sg.N;
-      const int buf = dbuf ? (iter & 1) : 0, use = dbuf ? (iter >> 1) : iter;
+      const int n0 = T.n0 + rank * 128, row0 = T.row0;
+      const int buf = iter & 1, use = iter >> 1;
       const uint32_t acc_empty = acc_empty0 + 8 * buf;
+      auto drained = [&]() {
+        tc_fence_before();
+        if (lane == 0) {
+          if (kPair) mbar_arrive_leader(acc_empty); else mbar_arrive(acc_empty);
+        }
+      };
       ok = __all_sync(0xffffffffu, mbar_wait_bounded(acc_full0 + 8 * buf, uint32_t(use & 1), abort_flag));
       if (!ok) {
         if (lane == 0 && P.status) atomicOr(P.status, B200RWKV_STATUS_WAIT_FULL);
         break;
       }
       tc_fence_after();
-      const int nchunks = Rt / CH, nitems = (two ? 2 : 1) * nchunks;
       int last_item = -1;     // this warp's last item that really reads TMEM
-      for (int item = eg; item < nitems; item += EG)
-        if (row0 + (item % nchunks) * CH < P.R) last_item = item;
-      if (last_item < 0) {
-        tc_fence_before();
-        if (lane == 0) mbar_arrive(acc_empty);
-      }
+      for (int item = eg; item < nchunks; item += EG)
+        if (row0 + item * CH < P.R) last_item = item;
+      if (last_item < 0) drained();
       const int rlast = P.R - 1;
       // rounding to the matrices' type, activation, gate, residual and store for 8 rows of one output column
-      auto finish = [&](const float (&acc)[CH], int h, int j0) {
-        const int n = n0 + h * 128 + q * 32 + lane;
+      auto finish = [&](const float (&acc)[CH], int j0) {
+        const int n = n0 + q * 32 + lane;
         const bool nvalid = n < Sg.N;
         const int nc = nvalid ? n : Sg.N - 1;
         float yv[CH];
@@ -273,25 +286,21 @@ __global__ void __launch_bounds__(kGemmThreads, 1) dense_tile_gemm_kernel(const 
           }
         }
       };
-      // K split: this slice's partial sums go to [tile][slice][row][128 weight rows] (mt = 128 only)
+      // K split: this slice's partial sums go to [tile][slice][row][128 weight rows] (single-CTA tiles only)
       float* sk = S > 1 ? P.sk_part + (size_t(tile) * S + slice) * Rt * 128 + q * 32 + lane : nullptr;
 #pragma unroll 1
-      for (int item = eg; item < nitems; item += EG) {
-        const int h = item / nchunks, j0 = (item - h * nchunks) * CH;
+      for (int item = eg; item < nchunks; item += EG) {
+        const int j0 = item * CH;
         if (row0 + j0 >= P.R) continue;   // warp-uniform
-        const uint32_t tbase = tmem + (uint32_t(q * 32) << 16) + uint32_t((h + buf) * kGemmAcc1Col + j0);
         int d[CH];
-        tmem_ld8(tbase, d);
+        tmem_ld8(tmem + (uint32_t(q * 32) << 16) + uint32_t(buf * kGemmAcc1Col + j0), d);
         tmem_ld_wait();
-        if (item == last_item) {
-          tc_fence_before();
-          if (lane == 0) mbar_arrive(acc_empty);
-        }
+        if (item == last_item) drained();
         float acc[CH];
 #pragma unroll
         for (int j = 0; j < CH; ++j) acc[j] = __int_as_float(d[j]);
         if (S == 1) {
-          finish(acc, h, j0);
+          finish(acc, j0);
         } else {
 #pragma unroll
           for (int j = 0; j < CH; ++j) sk[size_t(j0 + j) * 128] = acc[j];   // 32 lanes = 128 consecutive bytes per store
@@ -319,7 +328,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) dense_tile_gemm_kernel(const 
 #pragma unroll
               for (int j = 0; j < CH; ++j) acc[j] += __ldcg(all + (size_t(sl) * Rt + j0 + j) * 128);
             }
-            finish(acc, 0, j0);
+            finish(acc, j0);
           }
           if (et == 0) P.sk_count[tile] = 0u;              // leave the tickets zero for the next launch
         }
@@ -330,7 +339,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) dense_tile_gemm_kernel(const 
 
   tc_fence_before();
   __syncthreads();
-  if (tid == 0 && *abort_flag) {      // copies that may still be in flight into this CTA's shared memory
+  if (tid == 0 && rank == 0 && *abort_flag) {      // copies that may still be in flight into shared memory
     const int issued = *issued_ptr;
     const unsigned long long t0 = globaltimer_ns();
     for (int i = issued > NS ? issued - NS : 0; i < issued; ++i) {
@@ -339,9 +348,10 @@ __global__ void __launch_bounds__(kGemmThreads, 1) dense_tile_gemm_kernel(const 
       }
     }
   }
+  if (kPair) cluster_sync();             // nothing of the pair's work touches either CTA any more
   if (warp == 2) {
     tc_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kGemmTmemCols) : "memory");
+    tmem_dealloc<kPair>(tmem);
   }
 }
 

@@ -24,7 +24,7 @@
 // read the accumulators with tcgen05.ld and apply the affine terms and the fused element-wise op.
 // What bounds it: shared-memory traffic.  A K step writes (128 + 3*Rt) * 128 bytes by TMA and the MMAs
 // read every operand row again per 32 bytes of K.  Measured (7B ffn value, K = 16384, per K step and
-// CTA): single 80 rows 0.37 us, pair 160 rows 0.565 us, the MMAs alone 0.26 and 0.51 us at 1.87 GHz.
+// CTA): single 80 rows 0.345 us, pair 160 rows 0.555 us, the MMAs alone 0.26 and 0.51 us at 1.87 GHz.
 // L2 is not the limit (TMA boxes come from L2 at 16 to 19 TB/s in aggregate, 110 to 130 GB/s per SM).
 // Tiles that share a weight tile are adjacent in issue order so it is read from HBM once and from L2
 // afterwards.  The host picks the form, Rt and, for launches with too few tiles, a split of K over
@@ -83,7 +83,7 @@ struct GemmParams {
   int Rt;              // activation rows one CTA holds of a tile (multiple of 16, <= 80)
   int pair;            // tiles of a CTA pair: 256 weight rows x 2*Rt activation rows
   int dbuf;            // the accumulator has two buffers
-  int kc;              // 128-byte chunks of K per stage (one TMA copy each for the weights and the digits of a stage)
+  int kc;              // 128-byte chunks of K per stage, 1 or 2 (one TMA copy each for the weights and the digits of a stage)
   int stages;          // ring depth
   int stage_bytes;     // kc * (128 + 3*Rt) * 128, a multiple of 1024
   int row_tiles;       // ceil(R / activation rows per tile)
@@ -257,9 +257,9 @@ inline int gemm_block_tiles(int row_tiles, int rows_tile, int K) {
 }
 
 // 128-byte K chunks per stage.  One turn of the producer and of the MMA issuer (wait, copies or MMAs,
-// commit) costs about 0.2 us whatever it moves, so small tiles take two chunks per turn, where three
-// stages of them still fit the ring (two stages are slower than twice as many half as large).
-inline int gemm_chunks_per_stage(int chunk_bytes, int nk) { return nk >= 2 && 3 * 2 * chunk_bytes <= kGemmRingBytes ? 2 : 1; }
+// commit) costs about 0.2 us whatever it moves, so small tiles take two chunks per turn where the ring
+// still holds three stages of them, or four in a pair (fewer are slower than twice as many half as large).
+inline int gemm_chunks_per_stage(int chunk_bytes, int nk, bool pair) { return nk >= 2 && (pair ? 4 : 3) * 2 * chunk_bytes <= kGemmRingBytes ? 2 : 1; }
 
 // kPair: two CTAs of a cluster work on one tile with tcgen05.mma.cta_group::2 (see the file comment).
 template <bool kPair>
@@ -318,28 +318,29 @@ __global__ void __launch_bounds__(kGemmThreads, 1) tile_gemm_kernel(const __grid
       // Weights are constants: the first ring of them is requested before the launch dependency
       // resolves, while the preparation kernel in front of this launch still runs.  (An L2 prefetch of
       // 64 to 512 KB per CTA beyond the ring was no faster at any size, 5 % slower at few rows.)
-      struct Cursor { int it, k0; GemmTile T; };
-      auto start = [&](Cursor& c) { c.it = first_item; c.k0 = 0; if (c.it < nitems_all) c.T = gemm_tile(P, c.it / S); };
-      auto next = [&](Cursor& c) {
-        if ((c.k0 += KC) >= nk) {
-          c.k0 = 0;
-          if ((c.it += item_stride) < nitems_all) c.T = gemm_tile(P, c.it / S);
-        }
+      struct Cursor { int it, k, left; GemmTile T; };      // work item, K step of the copy, K steps left of the item
+      auto start = [&](Cursor& c) {
+        if (c.it < nitems_all) { c.T = gemm_tile(P, c.it / S); c.k = S == 1 ? 0 : (c.it % S) * nk; c.left = nk; }
       };
-      auto kstep = [&](const Cursor& c) { return (S == 1 ? 0 : (c.it % S) * nk) + c.k0; };
+      auto next = [&](Cursor& c) {
+        c.k += KC;
+        if ((c.left -= KC) <= 0) { c.it += item_stride; start(c); }
+      };
       Cursor ld;
+      ld.it = first_item;
       start(ld);
       int early = 0;
       for (; early < NS && ld.it < nitems_all; ++early, next(ld)) {
         if (elect_one()) {
           if (rank == 0) mbar_arrive_expect_tx(full0 + 8 * early, tx_bytes);
-          tma_operand_3d<kPair>(ring0 + uint32_t(early) * stage_bytes, &P.seg[ld.T.seg].wmap, 0, ld.T.n0 + rank * 128, kstep(ld), full_at + 8 * early);
+          tma_operand_3d<kPair>(ring0 + uint32_t(early) * stage_bytes, &P.seg[ld.T.seg].wmap, 0, ld.T.n0 + rank * 128, ld.k, full_at + 8 * early);
         }
       }
       *issued_ptr = early;
       griddep_wait();   // the digit rows come from the preparation kernel in front of this launch
       int issued = 0, slot = 0;
       uint32_t phase = 0;
+      ld.it = first_item;
       for (start(ld); ld.it < nitems_all; next(ld)) {
         const GemmSeg& Sg = P.seg[ld.T.seg];
         const uint32_t bar = full_at + 8 * slot, dst = ring0 + uint32_t(slot) * stage_bytes;
@@ -347,10 +348,10 @@ __global__ void __launch_bounds__(kGemmThreads, 1) tile_gemm_kernel(const __grid
           if (!warp_wait(empty0 + 8 * slot, phase ^ 1u, abort_flag, P.status, B200RWKV_STATUS_WAIT_EMPTY)) break;
           if (elect_one()) {
             if (rank == 0) mbar_arrive_expect_tx(full0 + 8 * slot, tx_bytes);
-            tma_operand_3d<kPair>(dst, &Sg.wmap, 0, ld.T.n0 + rank * 128, kstep(ld), bar);   // rows past N and chunks past K are zero-filled
+            tma_operand_3d<kPair>(dst, &Sg.wmap, 0, ld.T.n0 + rank * 128, ld.k, bar);   // rows past N and chunks past K are zero-filled
           }
         }
-        if (elect_one()) tma_operand_4d<kPair>(dst + a_bytes, &Sg.xmap, 0, ld.T.row0 + rank * Rt, 0, kstep(ld), bar);
+        if (elect_one()) tma_operand_4d<kPair>(dst + a_bytes, &Sg.xmap, 0, ld.T.row0 + rank * Rt, 0, ld.k, bar);
         ++issued;
         if (++slot == NS) { slot = 0; phase ^= 1u; }
       }
@@ -377,17 +378,23 @@ __global__ void __launch_bounds__(kGemmThreads, 1) tile_gemm_kernel(const __grid
           if (elect_one()) {
             tc_fence_after();
             const uint32_t a = ring0 + uint32_t(slot) * stage_bytes;
-            uint64_t ad = umma_desc(a), bd = umma_desc(a + a_bytes);
-            const int nc = min(KC, nk - k0);
-            for (int c = 0; c < nc; ++c) {
+            const uint64_t ad = umma_desc(a), bd = umma_desc(a + a_bytes);
+            // straight-line issue: a run-time loop around the MMAs costs more clocks than a small MMA takes
+            auto chunk = [&](uint64_t a64, uint64_t b64, uint32_t first) {
+              if (second) {
 #pragma unroll
-              for (int k = 0; k < 4; ++k) {   // 32 bytes of K per instruction: +2 in the descriptors' 16-byte address units
-                umma_i8<kPair>(tacc, ad + uint64_t(2 * k), bd + uint64_t(2 * k), idesc1, k == 0 && c == 0 ? acc : 1u);
-                if (second)
-                  umma_i8<kPair>(tmem + kGemmAcc1Col, ad + uint64_t(2 * k), bd + uint64_t(128 * 128 / 16 + 2 * k), idesc2, k == 0 && c == 0 ? acc : 1u);
+                for (int k = 0; k < 4; ++k) {   // 32 bytes of K per instruction: +2 in the descriptors' 16-byte address units
+                  umma_i8<kPair>(tacc, a64 + uint64_t(2 * k), b64 + uint64_t(2 * k), idesc1, k == 0 ? first : 1u);
+                  umma_i8<kPair>(tmem + kGemmAcc1Col, a64 + uint64_t(2 * k), b64 + uint64_t(128 * 128 / 16 + 2 * k), idesc2, k == 0 ? first : 1u);
+                }
+              } else {
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                  umma_i8<kPair>(tacc, a64 + uint64_t(2 * k), b64 + uint64_t(2 * k), idesc1, k == 0 ? first : 1u);
               }
-              ad += uint64_t(a_chunk >> 4); bd += uint64_t(b_chunk >> 4);
-            }
+            };
+            chunk(ad, bd, acc);
+            if (KC > 1 && nk - k0 > 1) chunk(ad + uint64_t(a_chunk >> 4), bd + uint64_t(b_chunk >> 4), 1u);
             umma_commit<kPair>(empty0 + 8 * slot);             // frees the stage (in both CTAs) once these MMAs have read it
             if (k0 + KC >= nk) umma_commit<kPair>(acc_full0 + 8 * buf);   // accumulators of this tile complete
           }
