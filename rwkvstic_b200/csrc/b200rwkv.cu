@@ -8,6 +8,7 @@
 
 #include "stream_gemv.cuh"
 #include "tile_gemm.cuh"
+#include "wkv_rows.cuh"
 #include "sampling.cuh"
 #include "dense_gemv.cuh"
 #include "decode_step.cuh"
@@ -364,141 +365,9 @@ embed_ln0_rows_kernel(const float* __restrict__ emb, const long long* __restrict
   for (int i = tid; i < D; i += 256) o[i] = w[i] * ((row[i] - mean) / sdev) + b[i];
 }
 
-// WKV-4 over rows laid out [stream][T][C]: one thread per (stream, channel), sequential over T,
-// max-trick state rows of stream s at aa/bb/pp + s * state_stride; y = gate * wkv written over k.
-__global__ void __launch_bounds__(128)
-wkv_rows_kernel(int B, int T, int C, const float* __restrict__ w, const float* __restrict__ u, float* __restrict__ k,
-                const float* __restrict__ v, const float* __restrict__ gate, float* __restrict__ aa,
-                float* __restrict__ bb, float* __restrict__ pp, long long state_stride) {
-  griddep_launch_dependents();
-  const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= B * C) return;
-  const int s = idx / C, c = idx - s * C;
-  const float wv = __ldg(w + c), uv = __ldg(u + c);
-  const size_t so = size_t(s) * state_stride + c;
-  // the state rows were last touched a whole step ago: on their way from DRAM while the GEMM in front still runs
-  asm volatile("prefetch.global.L2 [%0];" ::"l"(aa + so));
-  asm volatile("prefetch.global.L2 [%0];" ::"l"(bb + so));
-  asm volatile("prefetch.global.L2 [%0];" ::"l"(pp + so));
-  griddep_wait();
-  float a = aa[so], q = bb[so], p = pp[so];
-  const size_t base = size_t(s) * T * C + c;
-  // The recurrence is sequential in t but its inputs are not: fetch eight steps at a time so the
-  // chain waits for memory once per eight steps instead of once per step.
-  constexpr int U = 8;
-  int t = 0;
-  for (; t + U <= T; t += U) {
-    float kv[U], vv[U], gv[U];
-#pragma unroll
-    for (int i = 0; i < U; ++i) {
-      const size_t o = base + size_t(t + i) * C;
-      kv[i] = __ldcg(k + o); vv[i] = __ldcg(v + o); gv[i] = __ldcg(gate + o);
-    }
-#pragma unroll
-    for (int i = 0; i < U; ++i) k[base + size_t(t + i) * C] = gv[i] * wkv_step(kv[i], vv[i], wv, uv, a, q, p);
-  }
-  for (; t < T; ++t) {
-    const size_t o = base + size_t(t) * C;
-    k[o] = gate[o] * wkv_step(k[o], v[o], wv, uv, a, q, p);
-  }
-  aa[so] = a; bb[so] = q; pp[so] = p;
-}
-
-
-// ---- WKV over long rows: T cut into chunks that run in parallel (the recurrence is a scan whose
-// state composes: after n steps without input the max-trick state (aa, bb, pp) is (aa, bb, pp + n*w),
-// and two states add after bringing them to a common exponent).
-constexpr int kWkvChunk = 64;
-
-// Pass 1: thread (stream, chunk j, channel) runs chunk j from the EMPTY state and stores the
-// resulting local state (no outputs); the last chunk is not needed.  The thread of chunk 0 also
-// copies the stream's state into the scratch (behind the local states): pass 2 reads that snapshot,
-// because its last-chunk thread overwrites the state while the other chunks' threads may not have
-// started yet.
-__global__ void __launch_bounds__(128)
-wkv_chunk_state_kernel(int B, int T, int C, int NC, const float* __restrict__ w, const float* __restrict__ k,
-                       const float* __restrict__ v, float* __restrict__ loc, const float* __restrict__ aa,
-                       const float* __restrict__ bb, const float* __restrict__ pp, long long state_stride) {
-  griddep_launch_dependents();
-  griddep_wait();
-  const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= (long long)B * (NC - 1) * C) return;
-  const int c = int(idx % C);
-  const int j = int((idx / C) % (NC - 1)), s = int(idx / ((long long)C * (NC - 1)));
-  const float wv = w[c];
-  float a = 0.f, q = 0.f, p = -1e30f;
-  const size_t base = (size_t(s) * T + size_t(j) * kWkvChunk) * C + c;
-  constexpr int U = 8;
-  for (int t = 0; t < kWkvChunk; t += U) {   // chunks before the last are full
-    float kv[U], vv[U];
-#pragma unroll
-    for (int i = 0; i < U; ++i) { kv[i] = __ldcg(k + base + size_t(t + i) * C); vv[i] = __ldcg(v + base + size_t(t + i) * C); }
-#pragma unroll
-    for (int i = 0; i < U; ++i) {
-      const float ww2 = p + wv, p2 = fmaxf(ww2, kv[i]);
-      const float f1 = expf(ww2 - p2), f2 = expf(kv[i] - p2);
-      a = f1 * a + f2 * vv[i]; q = f1 * q + f2; p = p2;
-    }
-  }
-  float* o = loc + (size_t(s) * (NC - 1) + j) * 3 * C + c;
-  o[0] = a; o[size_t(C)] = q; o[2 * size_t(C)] = p;
-  if (j == 0) {
-    const size_t so = size_t(s) * state_stride + c;
-    float* snap = loc + (size_t(B) * (NC - 1) + s) * 3 * C + c;
-    snap[0] = aa[so]; snap[size_t(C)] = bb[so]; snap[2 * size_t(C)] = pp[so];
-  }
-}
-
-// Pass 2: thread (stream, chunk j, channel) rebuilds the state at the start of chunk j from the
-// stream's state and the local states of chunks 0..j-1, then runs chunk j with outputs
-// (y = gate * wkv written over k).  The thread of the last chunk stores the stream's new state.
-__global__ void __launch_bounds__(128)
-wkv_chunk_output_kernel(int B, int T, int C, int NC, const float* __restrict__ w, const float* __restrict__ u,
-                        float* __restrict__ k, const float* __restrict__ v, const float* __restrict__ gate,
-                        const float* __restrict__ loc, float* __restrict__ aa, float* __restrict__ bb,
-                        float* __restrict__ pp, long long state_stride) {
-  griddep_launch_dependents();
-  griddep_wait();
-  const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= (long long)B * NC * C) return;
-  const int c = int(idx % C);
-  const int j = int((idx / C) % NC), s = int(idx / ((long long)C * NC));
-  const float wv = w[c], uv = u[c];
-  const size_t so = size_t(s) * state_stride + c;
-  const float* snap = loc + (size_t(B) * (NC - 1) + s) * 3 * C + c;   // the state as pass 1 found it
-  float a = __ldcg(snap), q = __ldcg(snap + size_t(C)), p = __ldcg(snap + 2 * size_t(C));
-  const float wn = wv * float(kWkvChunk);
-  for (int i = 0; i < j; ++i) {
-    const float* l = loc + (size_t(s) * (NC - 1) + i) * 3 * C + c;
-    const float la = __ldcg(l), lq = __ldcg(l + size_t(C)), lp = __ldcg(l + 2 * size_t(C));
-    const float pd = p + wn, pm = fmaxf(pd, lp);
-    const float e1 = expf(pd - pm), e2 = expf(lp - pm);
-    a = e1 * a + e2 * la; q = e1 * q + e2 * lq; p = pm;
-  }
-  const int t0 = j * kWkvChunk, t1 = t0 + kWkvChunk < T ? t0 + kWkvChunk : T;
-  const size_t base = size_t(s) * T * C + c;
-  constexpr int U = 8;
-  int t = t0;
-  for (; t + U <= t1; t += U) {
-    float kv[U], vv[U], gv[U];
-#pragma unroll
-    for (int i = 0; i < U; ++i) {
-      const size_t o = base + size_t(t + i) * C;
-      kv[i] = __ldcg(k + o); vv[i] = __ldcg(v + o); gv[i] = __ldcg(gate + o);
-    }
-#pragma unroll
-    for (int i = 0; i < U; ++i) k[base + size_t(t + i) * C] = gv[i] * wkv_step(kv[i], vv[i], wv, uv, a, q, p);
-  }
-  for (; t < t1; ++t) {
-    const size_t o = base + size_t(t) * C;
-    k[o] = gate[o] * wkv_step(k[o], v[o], wv, uv, a, q, p);
-  }
-  if (j == NC - 1) { aa[so] = a; bb[so] = q; pp[so] = p; }
-}
-
 struct RowsWorkspace {
   int* status;
-  float *xa, *xb, *kb, *vb, *rb, *kk, *shift_new, *wkv_loc;
+  float *xa, *xb, *kb, *vb, *rb, *kk, *shift_new;
   int* sk_acc;
   unsigned* sk_count;
   signed char* digits;
@@ -522,7 +391,6 @@ static RowsWorkspace carve_rows(const b200rwkv_model* m, int B, int T, void* bas
   w.rb = reinterpret_cast<float*>(take(R * D * 4));
   w.kk = reinterpret_cast<float*>(take(R * F * 4));
   w.shift_new = reinterpret_cast<float*>(take(size_t(B) * D * 4));
-  w.wkv_loc = reinterpret_cast<float*>(take(size_t(B) * size_t((T + kWkvChunk - 1) / kWkvChunk) * 3 * D * 4));   // local chunk states
   w.sk_acc = reinterpret_cast<int*>(take(kSplitAccBytes));        // split-K scratch, zero between launches
   w.sk_count = reinterpret_cast<unsigned*>(take(size_t(kSplitMaxTiles) * 4));
   w.digits = reinterpret_cast<signed char*>(take(kDigits * Rpad * (3 * D > F ? 3 * D : F)));
@@ -564,6 +432,20 @@ static cudaError_t launch_clustered(int cluster, Kernel kernel, dim3 grid, dim3 
 template <typename Kernel, typename... Args>
 static cudaError_t launch_chained(Kernel kernel, dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
   return launch_clustered(1, kernel, grid, block, smem, stream, args...);
+}
+
+// WKV over T rows of B streams in one launch (wkv_rows.cuh); st: the block's state rows of stream 0.
+static cudaError_t launch_wkv(int B, int T, int C, const float* w, const float* u, float* k, const float* v, const float* gate, float* st,
+                              long long state_stride, unsigned short* out16, int is_bf16, cudaStream_t stream) {
+  WkvParams P;
+  memset(&P, 0, sizeof(P));
+  P.w = w; P.u = u; P.k = k; P.v = v; P.gate = gate;
+  P.aa = st + 2 * size_t(C); P.bb = st + 3 * size_t(C); P.pp = st + 4 * size_t(C);
+  P.state_stride = state_stride; P.out16 = out16; P.is_bf16 = is_bf16; P.T = T; P.C = C;
+  if (T == 1) return launch_chained(wkv_step_kernel, dim3((B * C + 127) / 128), dim3(128), 0, stream, P, B * C);
+  int warps;
+  wkv_span_shape(B, T, C, device_sms(), &warps, &P.steps);
+  return launch_chained(wkv_span_kernel, dim3(C / 32, B), dim3(warps * 32), 0, stream, P);
 }
 
 template <int NT, int MODE, int G>
@@ -1047,7 +929,7 @@ static int dense_step_impl(const b200rwkv_dense_model* m, int l0, int l1, const 
 // ---- unquantised weights: many rows ------------------------------------------------------------------
 struct DenseRowsWorkspace {
   int* status;
-  float *xa, *xb, *kb, *vb, *rb, *carry_new, *wkv_loc;
+  float *xa, *xb, *kb, *vb, *rb, *carry_new;
   unsigned short *t0, *t1, *t2, *kk, *hx;
   float* sk_part;        // partial sums of K slices (launches with few rows)
   unsigned* sk_count;    // their tickets, zero between launches
@@ -1068,7 +950,6 @@ static DenseRowsWorkspace dense_carve_rows(const b200rwkv_dense_model* m, int B,
   w.vb = reinterpret_cast<float*>(take(R * D * 4));
   w.rb = reinterpret_cast<float*>(take(R * D * 4));
   w.carry_new = reinterpret_cast<float*>(take(size_t(B) * D * 4));
-  w.wkv_loc = reinterpret_cast<float*>(take(size_t(B) * size_t((T + kWkvChunk - 1) / kWkvChunk) * 3 * D * 4));
   w.t0 = reinterpret_cast<unsigned short*>(take(Rpad * D * 2));
   w.t1 = reinterpret_cast<unsigned short*>(take(Rpad * D * 2));
   w.t2 = reinterpret_cast<unsigned short*>(take(Rpad * D * 2));
@@ -1757,22 +1638,8 @@ static int forward_rows_impl(const b200rwkv_model* m, const int64_t* tokens, flo
     { const b200rwkv_matrix* mp[3] = {&ly.att_key, &ly.att_value, &ly.att_receptance};
       if ((e = launch_tile_gemm(P, mp, ws.digits, s, &why)) != cudaSuccess) goto launch_failed; }
     // 2. WKV recurrence over each stream's rows; kb <- sigmoid(r) * wkv
-    why = "wkv_rows launch failed";
-    if (T <= 2 * kWkvChunk) {
-      e = launch_chained(wkv_rows_kernel, dim3((B * D + 127) / 128), dim3(128), 0, s, B, T, D, ly.time_decay, ly.time_first, ws.kb,
-                         (const float*)ws.vb, (const float*)ws.rb, st + 2 * size_t(D), st + 3 * size_t(D), st + 4 * size_t(D),
-                         (long long)state_stride);
-    } else {   // long rows: chunks of 64 steps in parallel, two passes
-      const int NC = (T + kWkvChunk - 1) / kWkvChunk;
-      const long long n1 = (long long)B * (NC - 1) * D, n2 = (long long)B * NC * D;
-      e = launch_chained(wkv_chunk_state_kernel, dim3((unsigned)((n1 + 127) / 128)), dim3(128), 0, s, B, T, D, NC, ly.time_decay,
-                         (const float*)ws.kb, (const float*)ws.vb, ws.wkv_loc, (const float*)(st + 2 * size_t(D)),
-                         (const float*)(st + 3 * size_t(D)), (const float*)(st + 4 * size_t(D)), (long long)state_stride);
-      if (e == cudaSuccess)
-        e = launch_chained(wkv_chunk_output_kernel, dim3((unsigned)((n2 + 127) / 128)), dim3(128), 0, s, B, T, D, NC, ly.time_decay,
-                           ly.time_first, ws.kb, (const float*)ws.vb, (const float*)ws.rb, (const float*)ws.wkv_loc,
-                           st + 2 * size_t(D), st + 3 * size_t(D), st + 4 * size_t(D), (long long)state_stride);
-    }
+    why = "wkv launch failed";
+    e = launch_wkv(B, T, D, ly.time_decay, ly.time_first, ws.kb, ws.vb, ws.rb, st, state_stride, nullptr, 0, s);
     if (e != cudaSuccess) goto launch_failed;
     // 3. attention output projection + residual -> xb
     memset(&Q, 0, sizeof(Q));
@@ -2037,27 +1904,10 @@ int b200rwkv_dense_forward_rows_layers(const b200rwkv_dense_model* m, int layer_
     { const void* w[3] = {ly.att_key, ly.att_value, ly.att_receptance};
       const unsigned short* x[3] = {ws.t0, ws.t1, ws.t2};
       B200_DR_CHECK(launch_dense_gemm(P, w, x, D, Rpad, s, &why), "key/value/receptance"); }
-    // 2. WKV recurrence over each stream's rows; kb <- sigmoid(r) * wkv
+    // 2. WKV recurrence over each stream's rows; t0 <- T(sigmoid(r) * wkv)
     why = "wkv launch";
-    if (T <= 2 * kWkvChunk) {
-      e = launch_chained(wkv_rows_kernel, dim3((B * D + 127) / 128), dim3(128), 0, s, B, T, D, ly.time_decay, ly.time_first, ws.kb,
-                         (const float*)ws.vb, (const float*)ws.rb, st + 2 * size_t(D), st + 3 * size_t(D), st + 4 * size_t(D),
-                         (long long)state_stride);
-    } else {
-      const int NC = (T + kWkvChunk - 1) / kWkvChunk;
-      const long long n1 = (long long)B * (NC - 1) * D, n2 = (long long)B * NC * D;
-      e = launch_chained(wkv_chunk_state_kernel, dim3((unsigned)((n1 + 127) / 128)), dim3(128), 0, s, B, T, D, NC, ly.time_decay,
-                         (const float*)ws.kb, (const float*)ws.vb, ws.wkv_loc, (const float*)(st + 2 * size_t(D)),
-                         (const float*)(st + 3 * size_t(D)), (const float*)(st + 4 * size_t(D)), (long long)state_stride);
-      if (e == cudaSuccess)
-        e = launch_chained(wkv_chunk_output_kernel, dim3((unsigned)((n2 + 127) / 128)), dim3(128), 0, s, B, T, D, NC, ly.time_decay,
-                           ly.time_first, ws.kb, (const float*)ws.vb, (const float*)ws.rb, (const float*)ws.wkv_loc,
-                           st + 2 * size_t(D), st + 3 * size_t(D), st + 4 * size_t(D), (long long)state_stride);
-    }
-    B200_DR_CHECK(e, "wkv");
+    B200_DR_CHECK(launch_wkv(B, T, D, ly.time_decay, ly.time_first, ws.kb, ws.vb, ws.rb, st, state_stride, ws.t0, bf, s), "wkv");
     // 3. attention output + residual -> xb
-    B200_DR_CHECK(launch_chained(dense_rows_cast_kernel, dim3(unsigned(std::min<long long>((long long)R * D / 4 / 256 + 1, 4096))), dim3(256), 0, s,
-                                 (const float*)ws.kb, ws.t0, (long long)R * D / 4, bf), "cast");
     memset(&P, 0, sizeof(P));
     P.nseg = 1; P.R = R; P.is_bf16 = bf; P.status = ws.status; P.sk_part = R <= kDgSplitMaxRows ? ws.sk_part : nullptr; P.sk_count = ws.sk_count;
     fill_dgemm_seg(P.seg[0], D, ws.xb, D, ACT_NONE, 0);

@@ -468,17 +468,4 @@ dense_rows_prep_kernel(const DRowsPrepParams P) {
   }
 }
 
-// fp32 rows -> rows of the matrices' 16-bit type (the cast in front of torch.py:162-164's matmul).
-__global__ void __launch_bounds__(256)
-dense_rows_cast_kernel(const float* __restrict__ in, unsigned short* __restrict__ out, long long n4, int is_bf16) {
-  griddep_launch_dependents();
-  griddep_wait();
-  for (long long i = blockIdx.x * 256ll + threadIdx.x; i < n4; i += (long long)gridDim.x * 256) {
-    const float4 v = __ldcg(reinterpret_cast<const float4*>(in) + i);
-    ushort4 o;
-    o.x = bits16(v.x, is_bf16); o.y = bits16(v.y, is_bf16); o.z = bits16(v.z, is_bf16); o.w = bits16(v.w, is_bf16);
-    reinterpret_cast<ushort4*>(out)[i] = o;
-  }
-}
-
 }  // namespace b200

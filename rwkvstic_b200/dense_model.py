@@ -300,7 +300,7 @@ class B200DenseRWKV:
                 else:
                     _lib.check(self._L.b200rwkv_dense_forward_rows(C.byref(self._cmodel), part.data_ptr(), B, tp, state.data_ptr(),
                                                                    state.stride(0), lp, ws.data_ptr(), ws.numel(), stream))
-                self.launch_count += 12 * self.n_layer + 3
+                self.launch_count += 7 * self.n_layer + 3
                 self._rows_status_src = ws
             self._queue_status(self._rows_status_src)
         return out

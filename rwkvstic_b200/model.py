@@ -379,10 +379,10 @@ class B200RWKV:
             raise ValueError(f"state must be [{self.n_layer},5,{self.n_embd}], got {tuple(state.shape)}")
         return state.to(device=self.device, dtype=torch.float32).contiguous()
 
-    def _rows_launches(self, tokens_per_stream: int) -> int:
+    def _rows_launches(self) -> int:
         """Kernels one rows-path call launches for its blocks: four preparation and four GEMM launches per
-        block plus the WKV scan (one kernel up to 128 tokens per stream, two passes beyond)."""
-        return (9 if tokens_per_stream <= 128 else 10) * self.n_layer
+        block plus the WKV scan."""
+        return 9 * self.n_layer
 
     def forward_rows(self, tokens: torch.Tensor, state: torch.Tensor) -> torch.Tensor:
         """Tensor-core path: ``tokens [B,T]`` int64, ``state [B,L,5,D]`` fp32 contiguous on the
@@ -428,7 +428,7 @@ class B200RWKV:
         _lib.check(self._L.b200rwkv_forward_rows(C.byref(self._cmodel), piece.data_ptr(), B, tp, state.data_ptr(),
                                                  state.stride(0), None if out is None else out.data_ptr(),
                                                  ws.data_ptr(), ws.numel(), stream))
-        self.launch_count += self._rows_launches(tp) + 1 + (2 if out is not None else 0)
+        self.launch_count += self._rows_launches() + 1 + (2 if out is not None else 0)
 
     def _queue_rows_status(self, ws: torch.Tensor) -> None:
         """Start a non-blocking copy of a rows workspace's status word to pinned host memory; the next
@@ -481,7 +481,7 @@ class B200RWKV:
                 ent["graph"] = g
             if ent["graph"] is not None:
                 ent["graph"].replay()
-                self.launch_count += self._rows_launches(1) + 3
+                self.launch_count += self._rows_launches() + 3
             else:
                 self._rows_call(ent["tok"], B, 1, state, ent["out"], ent["ws"])
             self._queue_rows_status(ent["ws"])
@@ -534,7 +534,7 @@ class B200RWKV:
             _lib.check(self._L.b200rwkv_forward_rows_stage(
                 C.byref(self._cmodel), None if tokens is None else tokens.data_ptr(), x.data_ptr(), B, T,
                 state.data_ptr(), state.stride(0), None if out is None else out.data_ptr(), ws.data_ptr(), ws.numel(), stream))
-            self.launch_count += self._rows_launches(T) + (1 if tokens is not None else 0) + (2 if want_logits else 0)
+            self.launch_count += self._rows_launches() + (1 if tokens is not None else 0) + (2 if want_logits else 0)
             self._last_rows_ws = ws
         return out
 
