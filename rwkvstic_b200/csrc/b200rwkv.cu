@@ -641,6 +641,33 @@ argmax_rows_kernel(const float* __restrict__ x, int n, long long ldx, long long*
   }
 }
 
+static cudaError_t launch_sample(const float* x, int rows, int n, long long ldx, float temp, float tau, const float* u, long long* out,
+                                 float* probs_out, long long* hist, int* hist_count, int hist_cap, cudaStream_t stream) {
+  static bool configured[64];
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
+  if (!configured[dev]) {
+    e = cudaFuncSetAttribute(sample_typical_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSampleMaxSlice * 4);
+    if (e != cudaSuccess) return e;
+    configured[dev] = true;
+  }
+  const int c = sample_cluster(rows, n, device_sms());
+  const int slice = (n + c - 1) / c;
+  const bool in_smem = slice <= kSampleMaxSlice;
+  cudaLaunchConfig_t cfg;
+  memset(&cfg, 0, sizeof(cfg));
+  cfg.gridDim = dim3(unsigned(rows) * unsigned(c)); cfg.blockDim = dim3(kSampleThreads); cfg.stream = stream;
+  cfg.dynamicSmemBytes = in_smem ? size_t(slice) * 4 : 0;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = unsigned(c); attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr; cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, in_smem ? sample_typical_kernel<true> : sample_typical_kernel<false>, x, n, ldx, temp, tau, u, out,
+                            probs_out, hist, hist_count, hist_cap, slice);
+}
+
 // ---------------------------------------------------------------------------------------- static scratch
 // Scratch of b200rwkv_gemv_u8_static: digit planes (up to kStaticPlaneBytes) followed by the
 // per-matrix scalars.  Lives in every GPU's memory from the moment the library is loaded there.
@@ -1733,10 +1760,8 @@ int b200rwkv_sample_typical(const float* x, int rows, int n, int64_t ldx, float 
   if (!x || !u || !out || rows < 1 || n < 1 || ldx < n || !(temp > 0.f) || !(tau > 0.f) ||
       (history && (!history_count || history_capacity < 1 || rows != 1)))
     return fail(B200RWKV_EINVAL, "sample_typical: bad argument (rows=%d n=%d temp=%g tau=%g)", rows, n, double(temp), double(tau));
-  sample_typical_kernel<<<rows, kSampleThreads, 0, static_cast<cudaStream_t>(stream)>>>(
-      x, n, ldx, temp, tau, u, reinterpret_cast<long long*>(out), probs_out, reinterpret_cast<long long*>(history),
-      history_count, history_capacity);
-  cudaError_t e = cudaGetLastError();
+  cudaError_t e = launch_sample(x, rows, n, ldx, temp, tau, u, reinterpret_cast<long long*>(out), probs_out,
+                                reinterpret_cast<long long*>(history), history_count, history_capacity, static_cast<cudaStream_t>(stream));
   if (e != cudaSuccess) return fail(B200RWKV_ECUDA, "sample_typical: %s", cudaGetErrorString(e));
   return B200RWKV_OK;
 }
