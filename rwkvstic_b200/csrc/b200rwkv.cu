@@ -453,6 +453,40 @@ static cudaError_t launch_rows_prep_as(const RowsPrepParams& P, dim3 grid, size_
   return launch_chained(rows_prep_kernel<NT, MODE, G>, grid, dim3(NT), smem, stream, P);
 }
 
+template <int NSEG, bool LN, int G, int NT_MAX, int MIN_CTAS>
+static cudaError_t launch_rows_stream_as(const RowsPrepParams& P, const RowsStreamShape& sh, cudaStream_t stream) {
+  static bool configured[64];
+  auto kernel = rows_stream_kernel<NSEG, LN, G, NT_MAX, MIN_CTAS>;
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
+  if (!configured[dev]) {
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit);
+    // the split between L1 and shared memory of the GEMM it alternates with (a change drains the SM first)
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+    if (e != cudaSuccess) return e;
+    configured[dev] = true;
+  }
+  return launch_chained(kernel, dim3(LN ? 1 : P.nseg, (P.R + P.rows_per_cta - 1) / P.rows_per_cta), dim3(sh.threads), sh.smem, stream, P);
+}
+
+template <int NSEG>
+static cudaError_t launch_rows_stream_ln(const RowsPrepParams& P, const RowsStreamShape& sh, cudaStream_t stream) {
+  if (sh.G == 2) return launch_rows_stream_as<NSEG, true, 2, 640, 1>(P, sh, stream);
+  if (sh.threads <= 640) return launch_rows_stream_as<NSEG, true, 1, 640, 2>(P, sh, stream);
+  return launch_rows_stream_as<NSEG, true, 1, 1024, 1>(P, sh, stream);
+}
+
+static cudaError_t launch_rows_stream(RowsPrepParams& P, const RowsStreamShape& sh, int sms, cudaStream_t stream) {
+  const int slots = sms * sh.slots_per_sm;
+  P.segs_per_cta = P.mode == ROWS_LN ? P.nseg : 1;
+  P.rows_per_cta = (P.R + slots - 1) / slots;
+  if (P.mode == ROWS_LN)
+    return P.nseg == 3 ? launch_rows_stream_ln<3>(P, sh, stream) : P.nseg == 2 ? launch_rows_stream_ln<2>(P, sh, stream) : launch_rows_stream_ln<1>(P, sh, stream);
+  return launch_rows_stream_as<1, false, 5, 1024, 1>(P, sh, stream);
+}
+
 static cudaError_t launch_rows_prep(const RowsPrepParams& P_in, cudaStream_t stream, const char** why) {
   static bool configured[64];
   static int sm_count[64];
@@ -468,6 +502,8 @@ static cudaError_t launch_rows_prep(const RowsPrepParams& P_in, cudaStream_t str
     configured[dev] = true;
   }
   RowsPrepParams P = P_in;
+  RowsStreamShape sh;
+  if (rows_stream_shape(P, &sh)) return launch_rows_stream(P, sh, sm_count[dev], stream);
   rows_prep_grouping(P.nseg, P.K, P.mode, P.R, sm_count[dev], &P.segs_per_cta, &P.rows_per_cta);
   const size_t smem = rows_prep_smem(P.K, P.mode);
   const int groups = (P.R + P.rows_per_cta - 1) / P.rows_per_cta;
@@ -1066,6 +1102,34 @@ static cudaError_t launch_dense_gemm(DGemmParams& P, const void* const* w, const
   int pair = 0, Rt = 16, ksplit = 1;
   if (!dense_gemm_pick_tile(P, K * 2 / 128, &pair, &Rt, &ksplit)) { *why = "no tile fits"; return cudaErrorInvalidValue; }
   return launch_dense_gemm_as(P, w, x, K, rows_alloc, pair != 0, Rt, ksplit, 0, stream, why);
+}
+
+template <int G, int NT_MAX, int MIN_CTAS>
+static cudaError_t launch_dense_rows_prep_as(const DRowsPrepParams& P, const DRowsShape& sh, cudaStream_t stream) {
+  static bool configured[64];
+  auto kernel = dense_rows_prep_kernel<G, NT_MAX, MIN_CTAS>;
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
+  if (!configured[dev]) {
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+    if (e != cudaSuccess) return e;
+    configured[dev] = true;
+  }
+  return launch_chained(kernel, dim3((P.R + P.rows_per_cta - 1) / P.rows_per_cta), dim3(sh.threads), sh.smem, stream, P);
+}
+
+static cudaError_t launch_dense_rows_prep(DRowsPrepParams& P, cudaStream_t stream) {
+  const DRowsShape sh = dense_rows_prep_shape(P.D, P.nmix);
+  // one row per CTA while that fits the GPU at once; beyond, a CTA walks consecutive rows and takes each layer norm once
+  const int slots = std::max(device_sms(), 1) * sh.slots_per_sm;
+  P.rows_per_cta = (P.R + slots - 1) / slots;
+  P.hold_ln = sh.hold_ln;
+  if (sh.G == 1) return sh.threads <= 768 ? launch_dense_rows_prep_as<1, 768, 2>(P, sh, stream) : launch_dense_rows_prep_as<1, 1024, 1>(P, sh, stream);
+  if (sh.G == 2) return launch_dense_rows_prep_as<2, 1024, 1>(P, sh, stream);
+  return launch_dense_rows_prep_as<3, 1024, 1>(P, sh, stream);
 }
 
 static void fill_dgemm_seg(DGemmSeg& s, int N, void* out, long long ldo, int act, int out_t) {
@@ -1868,21 +1932,6 @@ int b200rwkv_dense_forward_rows_layers(const b200rwkv_dense_model* m, int layer_
   const char* why = "";
   cudaError_t e;
   g_chain_rows = R <= 1024;
-  static bool prep_configured[64];
-  static int prep_sms[64];
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return fail(B200RWKV_ECUDA, "dense_forward_rows: no current device");
-  if (!prep_configured[dev]) {
-    if (cudaFuncSetAttribute(dense_rows_prep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * kDsMaxEmbd * 4) != cudaSuccess ||
-        cudaDeviceGetAttribute(&prep_sms[dev], cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-      return fail(B200RWKV_ECUDA, "dense_forward_rows: cannot size the preparation kernel's shared memory");
-    prep_configured[dev] = true;
-  }
-  // preparation CTAs resident at once (registers, and two rows of shared memory each)
-  int prep_per_sm = 1;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&prep_per_sm, dense_rows_prep_kernel, 256, size_t(2) * D * 4) != cudaSuccess || prep_per_sm < 1)
-    prep_per_sm = 1;
-  const int prep_slots = prep_sms[dev] * prep_per_sm;
 #define B200_DR_CHECK(call, what)                                                                      \
   do {                                                                                                 \
     e = (call);                                                                                        \
@@ -1895,6 +1944,7 @@ int b200rwkv_dense_forward_rows_layers(const b200rwkv_dense_model* m, int layer_
                                  D, V, m->ln0_w, m->ln0_b, ws.xa), "embedding");
   DRowsPrepParams Q;
   DGemmParams P;
+  float* parked = nullptr;       // state row (of stream 0) that the parked carries belong to
   auto prep = [&](const float* x, const float* lw, const float* lb, const float* carry, int nmix, const float* const* mix,
                   unsigned short* const* out, int last_only) -> cudaError_t {
     memset(&Q, 0, sizeof(Q));
@@ -1903,15 +1953,12 @@ int b200rwkv_dense_forward_rows_layers(const b200rwkv_dense_model* m, int layer_
     Q.carry_out_stride = T == 1 ? state_stride : D;
     Q.nmix = nmix; Q.D = D; Q.Tn = T; Q.last_only = last_only; Q.is_bf16 = bf;
     for (int i = 0; i < (nmix > 0 ? nmix : 1); ++i) { Q.mix[i] = mix ? mix[i] : nullptr; Q.out[i] = out[i]; }
-    // one row per CTA while that fits the GPU at once; beyond, a CTA walks consecutive rows and takes each layer norm once
+    // more than one row per stream: the new carry is parked in ws.carry_new and goes to its state row with the
+    // next preparation launch (or the copy at the end of the call)
+    if (T > 1) { Q.commit_src = parked ? ws.carry_new : nullptr; Q.commit_dst = parked; }
+    parked = T > 1 && carry ? const_cast<float*>(carry) : nullptr;
     Q.R = last_only ? B : R;
-    Q.rows_per_cta = (Q.R + prep_slots - 1) / prep_slots;
-    return launch_chained(dense_rows_prep_kernel, dim3((Q.R + Q.rows_per_cta - 1) / Q.rows_per_cta), dim3(256), size_t(2) * D * 4, s, Q);
-  };
-  auto commit = [&](float* row) -> cudaError_t {      // parked layer norm of every stream's last row -> its state row
-    if (T == 1) return cudaSuccess;                    // one row per stream: the preparation kernel wrote the state row itself
-    return cudaMemcpy2DAsync(row, size_t(state_stride) * 4, ws.carry_new, size_t(D) * 4, size_t(D) * 4, size_t(B),
-                             cudaMemcpyDeviceToDevice, s);
+    return launch_dense_rows_prep(Q, s);
   };
   for (int l = layer_begin; l < layer_end; ++l) {
     const b200rwkv_dense_layer& ly = m->layers[l];
@@ -1920,7 +1967,6 @@ int b200rwkv_dense_forward_rows_layers(const b200rwkv_dense_model* m, int layer_
     { const float* mix[3] = {ly.att_mix_k, ly.att_mix_v, ly.att_mix_r};
       unsigned short* out[3] = {ws.t0, ws.t1, ws.t2};
       B200_DR_CHECK(prep(ws.xa, ly.ln1_w, ly.ln1_b, st, 3, mix, out, 0), "attention mix"); }
-    B200_DR_CHECK(commit(st), "attention carry");
     memset(&P, 0, sizeof(P));
     P.nseg = 3; P.R = R; P.is_bf16 = bf; P.status = ws.status; P.sk_part = R <= kDgSplitMaxRows ? ws.sk_part : nullptr; P.sk_count = ws.sk_count;
     fill_dgemm_seg(P.seg[0], D, ws.kb, D, ACT_NONE, 0);
@@ -1944,7 +1990,6 @@ int b200rwkv_dense_forward_rows_layers(const b200rwkv_dense_model* m, int layer_
     { const float* mix[2] = {ly.ffn_mix_k, ly.ffn_mix_r};
       unsigned short* out[2] = {ws.t0, ws.t1};
       B200_DR_CHECK(prep(ws.xb, ly.ln2_w, ly.ln2_b, st + D, 2, mix, out, 0), "ffn mix"); }
-    B200_DR_CHECK(commit(st + D), "ffn carry");
     memset(&P, 0, sizeof(P));
     P.nseg = 2; P.R = R; P.is_bf16 = bf; P.status = ws.status; P.sk_part = R <= kDgSplitMaxRows ? ws.sk_part : nullptr; P.sk_count = ws.sk_count;
     fill_dgemm_seg(P.seg[0], F, ws.kk, F, ACT_RELUSQ, 1);
@@ -1971,6 +2016,9 @@ int b200rwkv_dense_forward_rows_layers(const b200rwkv_dense_model* m, int layer_
     const unsigned short* x[1] = {ws.hx};
     B200_DR_CHECK(launch_dense_gemm(P, w, x, D, gemm_padded_rows(B), s, &why), "head");
   }
+  if (parked)
+    B200_DR_CHECK(cudaMemcpy2DAsync(parked, size_t(state_stride) * 4, ws.carry_new, size_t(D) * 4, size_t(D) * 4, size_t(B),
+                                    cudaMemcpyDeviceToDevice, s), "ffn carry");
 #undef B200_DR_CHECK
   return B200RWKV_OK;
 }

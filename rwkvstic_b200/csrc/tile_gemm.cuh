@@ -683,14 +683,14 @@ __device__ __forceinline__ void rows_store_digits(uint32_t* da, uint32_t* db, ui
     // round to nearest even of the fp32 product, sign included (|v * inv| <= kQMax < 2^23): one conversion
     // instead of the five instructions of the magnitude-and-sign form, same integer
     const int X = __float2int_rn(__fmul_rn(v[i], inv));
-    y[i] = uint32_t(X + 0x8080) ^ 0x8080u;   // bytes: (c, b, a, sign extension)
+    y[i] = uint32_t(X + 0x8080);   // bytes: (c + 128, b + 128, a, sign extension)
   }
   const uint32_t c01 = __byte_perm(y[0], y[1], 0x0040), c23 = __byte_perm(y[2], y[3], 0x0040);
   const uint32_t b01 = __byte_perm(y[0], y[1], 0x0051), b23 = __byte_perm(y[2], y[3], 0x0051);
   const uint32_t a01 = __byte_perm(y[0], y[1], 0x0062), a23 = __byte_perm(y[2], y[3], 0x0062);
   da[g] = __byte_perm(a01, a23, 0x5410);
-  db[g] = __byte_perm(b01, b23, 0x5410);
-  dc[g] = __byte_perm(c01, c23, 0x5410);
+  db[g] = __byte_perm(b01, b23, 0x5410) ^ 0x80808080u;
+  dc[g] = __byte_perm(c01, c23, 0x5410) ^ 0x80808080u;
 }
 
 __device__ __forceinline__ float4 ln_apply(float4 x, float mean, float rstd, float4 w, float4 b) {
@@ -1052,5 +1052,237 @@ inline void rows_prep_grouping(int nseg, int K, int mode, int R, int sms, int* s
   if ((long long)nseg * R <= 2 * slots) return;
   *segs_per_cta = nseg;
   *rows_per_cta = int((R + slots - 1) / slots);
+}
+
+// ---- streaming form: the usual matrices (no per-output terms, so no sums beside zp), rows of up to
+// 20480 inputs (5120 with the layer norm).  A thread owns the same 4*G inputs of every row it meets, so the
+// parameter vectors of all the launch's matrices are fetched once, before the launch dependency resolves,
+// and stay in the thread's own slots of shared memory; the next row is requested before this one is worked
+// on; all matrices of a row share one reduction (three barriers a row with the layer norm, one without).
+// What bounds it: instruction issue with thousands of rows, the chain of one row with few.  Against
+// rows_prep_kernel (parameters re-read for every matrix and row, each matrix reduced by itself), us:
+// three matrices, 4096 rows of 2560 inputs 78 -> 68, 256 rows of 4096 inputs 18 -> 15; two matrices 61 -> 51 and
+// 18 -> 12.  With mix and ry in registers a CTA had the SM to itself (20 warps of 2560 inputs): 88 us.
+// A row's arithmetic depends on K and the mode alone, not on how rows are dealt to CTAs.
+constexpr int kStreamGroupsMax = 5;
+constexpr int kStreamRedBytes = 2 * 8 * 32 * 4;     // two phases of up to eight values of 32 warps
+
+// Totals over the CTA, in every thread, of NV values: the first NMAX are maxima of non-negative numbers
+// (ordered like their bits), the rest sums.  Phases as in span_reduce.
+template <int NV, int NMAX>
+__device__ __forceinline__ void stream_reduce(float (&v)[NV], float* red, int& phase, int nwarps) {
+  static_assert(NV <= 8, "kStreamRedBytes");
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+  for (int k = 0; k < NV; ++k)
+    v[k] = k < NMAX ? __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(v[k]))) : warp_sum(v[k]);
+  float* slots = red + phase * 256;
+  phase ^= 1;
+  if (lane == 0) {
+#pragma unroll
+    for (int k = 0; k < NV; ++k) slots[k * 32 + warp] = v[k];
+  }
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < NV; ++k) {
+    const float t = lane < nwarps ? slots[k * 32 + lane] : 0.f;
+    v[k] = k < NMAX ? __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(t))) : warp_sum(t);
+  }
+}
+
+// NSEG matrices of one layer-normed row (mixed with the row before when NSEG > 1; NSEG = 1 is the head), or
+// (LN = false) the one matrix blockIdx.x of a plain input.  CTA blockIdx.y takes rows_per_cta rows.
+template <int NSEG, bool LN, int G, int NT_MAX, int MIN_CTAS>
+__global__ void __launch_bounds__(NT_MAX, MIN_CTAS) rows_stream_kernel(const __grid_constant__ RowsPrepParams P) {
+  extern __shared__ __align__(128) unsigned char prep_smem[];
+  constexpr bool kMix = LN && NSEG > 1;
+  constexpr int kRy = LN ? 2 : 0, kMy = kRy + NSEG, kMu = kMy + NSEG;     // held vectors: (ln w, b,) ry.., my.., (mix..)
+  float* red = reinterpret_cast<float*>(prep_smem);
+  float4* held = reinterpret_cast<float4*>(prep_smem + kStreamRedBytes);
+  const int tid = threadIdx.x, lane = tid & 31, NT = blockDim.x, nwarps = NT >> 5;
+  const int K = P.K, NG = K / 4;
+  const int sp = LN ? 0 : int(blockIdx.x);                   // plain: the matrix
+  const int r0 = int(blockIdx.y) * P.rows_per_cta, r1 = min(r0 + P.rows_per_cta, P.R);
+  const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
+  const float invk = 1.0f / float(K);
+  auto mine = [&](int g) { return G == 1 || g < NG; };       // one group: as many threads as groups
+  griddep_launch_dependents();
+
+#pragma unroll
+  for (int i = 0; i < G; ++i) {
+    const int g = tid + i * NT;
+    if (mine(g)) {
+      if (LN) {
+        const float4 w = ld_param_v4(reinterpret_cast<const float4*>(P.ln_w) + g), b = ld_param_v4(reinterpret_cast<const float4*>(P.ln_b) + g);
+        held[g] = w; held[NG + g] = b;
+      }
+#pragma unroll
+      for (int s = 0; s < NSEG; ++s) {
+        const PrepSeg& S = P.seg[LN ? s : sp];
+        const float4 ry = ld_param_v4(reinterpret_cast<const float4*>(S.ry) + g), my = ld_param_v4(reinterpret_cast<const float4*>(S.my) + g);
+        if constexpr (kMix) held[(kMu + s) * NG + g] = ld_param_v4(reinterpret_cast<const float4*>(S.mix) + g);
+        held[(kRy + s) * NG + g] = ry;
+        held[(kMy + s) * NG + g] = my;
+      }
+    }
+  }
+  griddep_wait();
+
+  const float* in = LN ? P.ln_x : P.seg[sp].xin;
+  auto load_row = [&](int r, float4 (&x)[G]) {
+    const float4* p = reinterpret_cast<const float4*>(in + size_t(r) * P.ldx);
+#pragma unroll
+    for (int i = 0; i < G; ++i) {
+      const int g = tid + i * NT;
+      x[i] = mine(g) ? __ldcg(p + g) : zero4;
+    }
+  };
+  float4 x[G], nx[G], pv[kMix ? G : 1];
+  int phase = 0;
+  int b = r0 / P.T, t = r0 - b * P.T;
+  load_row(r0, x);
+  bool fetch_prev = kMix && t > 0;              // this CTA's first row continues a stream: its predecessor is normed beside it
+  if constexpr (kMix) {
+    if (fetch_prev) load_row(r0 - 1, pv);
+  }
+
+  for (int r = r0; r < r1; ++r) {
+    if (r + 1 < r1) load_row(r + 1, nx);
+    if (P.commit_n > 0 && sp == 0 && t == P.T - 1) {
+      const float4* src = reinterpret_cast<const float4*>(P.commit_src + size_t(b) * P.commit_n);
+      float4* dst = reinterpret_cast<float4*>(P.commit_dst + size_t(b) * P.commit_stride);
+      for (int g = tid; g < P.commit_n / 4; g += NT) dst[g] = __ldcg(src + g);
+    }
+    if constexpr (LN) {
+      if constexpr (kMix) {
+        if (t == 0) {
+          const float4* carry = P.shift ? reinterpret_cast<const float4*>(P.shift + size_t(b) * P.shift_stride) : nullptr;
+#pragma unroll
+          for (int i = 0; i < G; ++i) {
+            const int g = tid + i * NT;
+            pv[i] = carry && mine(g) ? __ldcg(carry + g) : zero4;
+          }
+        }
+      }
+      // mean, then the sum of squared deviations (the centred form, see rows_prep_span)
+      auto norm = [&](float4 (&a)[G]) {
+        float s[1] = {0.f};
+#pragma unroll
+        for (int i = 0; i < G; ++i) s[0] += (a[i].x + a[i].y) + (a[i].z + a[i].w);      // groups past the end hold zeros
+        stream_reduce<1, 0>(s, red, phase, nwarps);
+        const float mean = s[0] * invk;
+        float q[1] = {0.f};
+#pragma unroll
+        for (int i = 0; i < G; ++i)
+          if (mine(tid + i * NT)) {
+            const float a0 = a[i].x - mean, a1 = a[i].y - mean, a2 = a[i].z - mean, a3 = a[i].w - mean;
+            q[0] += (a0 * a0 + a1 * a1) + (a2 * a2 + a3 * a3);
+          }
+        stream_reduce<1, 0>(q, red, phase, nwarps);
+        const float rstd = 1.0f / sqrtf(q[0] * invk + 1e-5f);
+#pragma unroll
+        for (int i = 0; i < G; ++i) {
+          const int g = tid + i * NT;
+          if (mine(g)) a[i] = ln_apply(a[i], mean, rstd, held[g], held[NG + g]);
+        }
+      };
+      if constexpr (kMix) {
+        if (fetch_prev) { norm(pv); fetch_prev = false; }
+      }
+      norm(x);
+      if (P.shift_out && t == P.T - 1) {
+#pragma unroll
+        for (int i = 0; i < G; ++i) {
+          const int g = tid + i * NT;
+          if (mine(g)) reinterpret_cast<float4*>(P.shift_out + size_t(b) * K)[g] = x[i];
+        }
+      }
+    }
+    // scaled inputs of every matrix, with max |xs| and sum v * my
+    float4 xs[NSEG][G];
+    float st[2 * NSEG];
+#pragma unroll
+    for (int s = 0; s < NSEG; ++s) {
+      float amax = 0.f, zp = 0.f;
+#pragma unroll
+      for (int i = 0; i < G; ++i) {
+        const int g = tid + i * NT;
+        if (mine(g)) {
+          float4 v = x[i];
+          if constexpr (kMix) {
+            const float4 m = held[(kMu + s) * NG + g], tc = pv[i];
+            v.x = x[i].x * m.x + tc.x * (1.f - m.x);
+            v.y = x[i].y * m.y + tc.y * (1.f - m.y);
+            v.z = x[i].z * m.z + tc.z * (1.f - m.z);
+            v.w = x[i].w * m.w + tc.w * (1.f - m.w);
+          }
+          const float4 ry = held[(kRy + s) * NG + g], my = held[(kMy + s) * NG + g];
+          const float4 y = make_float4(v.x * ry.x, v.y * ry.y, v.z * ry.z, v.w * ry.w);
+          amax = fmaxf(amax, fmaxf(fmaxf(fabsf(y.x), fabsf(y.y)), fmaxf(fabsf(y.z), fabsf(y.w))));
+          zp += (v.x * my.x + v.y * my.y) + (v.z * my.z + v.w * my.w);
+          xs[s][i] = y;
+        }
+      }
+      st[s] = amax; st[NSEG + s] = zp;
+    }
+    stream_reduce<2 * NSEG, NSEG>(st, red, phase, nwarps);
+    // lane s divides for matrix s
+    float amax = st[0], zp = st[NSEG];
+#pragma unroll
+    for (int s = 1; s < NSEG; ++s)
+      if (lane == s) { amax = st[s]; zp = st[NSEG + s]; }
+    const float inv = amax > 0.f ? kQMax / amax : 0.f;
+    if (tid < NSEG) {
+      SegScalars sc;
+      sc.sd = amax > 0.f ? __fdiv_rn(1.0f, inv) : 0.f;
+      sc.zp = zp; sc.sumxs = 0.f; sc.sumx = 0.f;
+      sc.pad[0] = sc.pad[1] = sc.pad[2] = sc.pad[3] = 0.f;
+      P.scal[size_t(LN ? tid : sp) * P.R + r] = sc;
+    }
+#pragma unroll
+    for (int s = 0; s < NSEG; ++s) {
+      const float is = __shfl_sync(0xffffffffu, inv, s);
+      const size_t plane = size_t(P.Rpad) * K;
+      signed char* d = P.digits + size_t((LN ? s : sp) * kDigits) * plane + size_t(r) * K;
+#pragma unroll
+      for (int i = 0; i < G; ++i) {
+        const int g = tid + i * NT;
+        if (mine(g))
+          rows_store_digits(reinterpret_cast<uint32_t*>(d), reinterpret_cast<uint32_t*>(d + plane), reinterpret_cast<uint32_t*>(d + 2 * plane), g, xs[s][i], is);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < G; ++i) {
+      if constexpr (kMix) pv[i] = x[i];
+      x[i] = nx[i];
+    }
+    if (++t == P.T) { t = 0; ++b; }
+  }
+}
+
+// Whether a launch takes the streaming form, and its shape: the fewest groups per thread that a CTA of 1024
+// threads allows (640 with two groups of a layer-normed row: their registers).  Plain rows take it only where
+// they are too long for the registers of rows_prep_kernel (K > 16384);
+// shorter ones have one reduction and two parameter vectors, and many small CTAs hide their latency better
+// (4096 rows of 2560 inputs 23 us against 26, of 10240 inputs 61 against 87).
+struct RowsStreamShape { int G, threads, slots_per_sm; size_t smem; };
+inline bool rows_stream_shape(const RowsPrepParams& P, RowsStreamShape* sh) {
+  if (P.need_sums) return false;
+  const bool ln = P.mode == ROWS_LN;
+  if (!ln && rows_prep_in_regs(P.K, P.mode, rows_prep_threads(P.K, P.mode))) return false;
+  if (ln)
+    for (int s = 0; s < P.nseg; ++s)
+      if ((P.seg[s].mix != nullptr) != (P.nseg > 1)) return false;
+  const int NG = P.K / 4;
+  sh->G = (NG + 1023) / 1024;
+  if (sh->G > (ln ? 2 : kStreamGroupsMax)) return false;
+  sh->threads = ((NG + sh->G - 1) / sh->G + 31) / 32 * 32;
+  if (ln && sh->G == 2 && sh->threads > 640) return false;
+  const int vectors = ln ? 2 + P.nseg * (P.nseg > 1 ? 3 : 2) : 2;
+  sh->smem = size_t(kStreamRedBytes) + size_t(vectors) * P.K * 4;
+  // resident CTAs: registers (48 a thread up to 640 threads, 64 above) and shared memory
+  const int by_threads = sh->G == 1 && sh->threads <= 640 ? 1280 / sh->threads : 1, by_smem = int(size_t(228 * 1024) / (sh->smem + 1024));
+  sh->slots_per_sm = by_threads < by_smem ? by_threads : by_smem;
+  return sh->slots_per_sm >= 1 && sh->smem <= size_t(kSmemLimit);
 }
 }  // namespace b200
