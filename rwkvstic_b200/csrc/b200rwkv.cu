@@ -484,7 +484,11 @@ static cudaError_t launch_rows_stream(RowsPrepParams& P, const RowsStreamShape& 
   P.rows_per_cta = (P.R + slots - 1) / slots;
   if (P.mode == ROWS_LN)
     return P.nseg == 3 ? launch_rows_stream_ln<3>(P, sh, stream) : P.nseg == 2 ? launch_rows_stream_ln<2>(P, sh, stream) : launch_rows_stream_ln<1>(P, sh, stream);
-  return launch_rows_stream_as<1, false, 5, 1024, 1>(P, sh, stream);
+  switch (sh.G) {
+    case 2: return launch_rows_stream_as<1, false, 2, 1024, 1>(P, sh, stream);
+    case 3: return launch_rows_stream_as<1, false, 3, 1024, 1>(P, sh, stream);
+    default: return launch_rows_stream_as<1, false, 5, 1024, 1>(P, sh, stream);
+  }
 }
 
 static cudaError_t launch_rows_prep(const RowsPrepParams& P_in, cudaStream_t stream, const char** why) {

@@ -1260,28 +1260,32 @@ __global__ void __launch_bounds__(NT_MAX, MIN_CTAS) rows_stream_kernel(const __g
   }
 }
 
-// Whether a launch takes the streaming form, and its shape: the fewest groups per thread that a CTA of 1024
-// threads allows (640 with two groups of a layer-normed row: their registers).  Plain rows take it only where
-// they are too long for the registers of rows_prep_kernel (K > 16384);
-// shorter ones have one reduction and two parameter vectors, and many small CTAs hide their latency better
-// (4096 rows of 2560 inputs 23 us against 26, of 10240 inputs 61 against 87).
+// Whether a launch takes the streaming form, and its shape.  Layer-normed rows: the fewest groups per thread that
+// a CTA of 1024 threads allows (two: at most 640 threads, for their registers).  Plain rows: the fewest from two up
+// that 512 threads allow, so that several CTAs share an SM, up to three groups (4096 rows of 2560 inputs 23 -> 21.6
+// us, 26 with one group and two CTAs; 256 rows of 4096 inputs 9.4 -> 7.9); rows of four groups and more stay with
+// rows_prep_kernel (4096 rows of 10240 inputs 61 us, 86 here: the row requested ahead leaves too few registers)
+// unless they are beyond its registers (K > 16384), where the alternative re-reads the row for every pass.
 struct RowsStreamShape { int G, threads, slots_per_sm; size_t smem; };
 inline bool rows_stream_shape(const RowsPrepParams& P, RowsStreamShape* sh) {
   if (P.need_sums) return false;
   const bool ln = P.mode == ROWS_LN;
-  if (!ln && rows_prep_in_regs(P.K, P.mode, rows_prep_threads(P.K, P.mode))) return false;
   if (ln)
     for (int s = 0; s < P.nseg; ++s)
       if ((P.seg[s].mix != nullptr) != (P.nseg > 1)) return false;
   const int NG = P.K / 4;
-  sh->G = (NG + 1023) / 1024;
+  sh->G = ln ? (NG + 1023) / 1024 : std::max(2, (NG + 511) / 512);
+  if (!ln && sh->G > 3) {
+    if (rows_prep_in_regs(P.K, P.mode, rows_prep_threads(P.K, P.mode))) return false;
+    sh->G = (NG + 1023) / 1024;
+  }
   if (sh->G > (ln ? 2 : kStreamGroupsMax)) return false;
   sh->threads = ((NG + sh->G - 1) / sh->G + 31) / 32 * 32;
   if (ln && sh->G == 2 && sh->threads > 640) return false;
   const int vectors = ln ? 2 + P.nseg * (P.nseg > 1 ? 3 : 2) : 2;
   sh->smem = size_t(kStreamRedBytes) + size_t(vectors) * P.K * 4;
   // resident CTAs: registers (48 a thread up to 640 threads, 64 above) and shared memory
-  const int by_threads = sh->G == 1 && sh->threads <= 640 ? 1280 / sh->threads : 1, by_smem = int(size_t(228 * 1024) / (sh->smem + 1024));
+  const int by_threads = ln ? (sh->G == 1 && sh->threads <= 640 ? 1280 / sh->threads : 1) : 1024 / sh->threads, by_smem = int(size_t(228 * 1024) / (sh->smem + 1024));
   sh->slots_per_sm = by_threads < by_smem ? by_threads : by_smem;
   return sh->slots_per_sm >= 1 && sh->smem <= size_t(kSmemLimit);
 }
