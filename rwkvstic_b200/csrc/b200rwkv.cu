@@ -1677,9 +1677,10 @@ static int forward_rows_impl(const b200rwkv_model* m, const int64_t* tokens, flo
   const char* why = "";
   cudaError_t e;
 
-  // Chaining pays when the kernels are short (decode, short prompts: 10-15 % per step); with thousands
-  // of rows per launch it measured 9 % slower than plain stream order (3B shape, 4096 rows), so it is off there.
-  g_chain_rows = B * T <= 1024;
+  // Chained at every size: the next launch's weights and parameters are requested while this one still runs
+  // (decode and short prompts 10-15 % per step; bf16 3B 2 x 701 tokens 10598 -> 10154 us, uint8 3B 8 x 1024 tokens,
+  // 4096 rows a call, 71868 -> 71569, within the noise).
+  g_chain_rows = true;
   if (x_ext) ws.xa = x_ext;
   if (tokens) {
     e = launch_chained(embed_ln0_rows_kernel, dim3(R), dim3(256), 0, s, m->emb, reinterpret_cast<const long long*>(tokens), D, V,
@@ -1935,7 +1936,7 @@ int b200rwkv_dense_forward_rows_layers(const b200rwkv_dense_model* m, int layer_
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const char* why = "";
   cudaError_t e;
-  g_chain_rows = R <= 1024;
+  g_chain_rows = true;
 #define B200_DR_CHECK(call, what)                                                                      \
   do {                                                                                                 \
     e = (call);                                                                                        \
