@@ -26,6 +26,8 @@
 
 #include <cooperative_groups.h>
 
+#include <utility>
+
 #include "common.cuh"
 
 namespace b200 {
@@ -120,6 +122,7 @@ sample_typical_kernel(const float* __restrict__ x, int n, long long ldx, float t
   __shared__ SampleShared S;
   namespace cg = cooperative_groups;
   const cg::cluster_group cluster = cg::this_cluster();
+  auto started = cluster.barrier_arrive();     // met before the first access to another CTA's memory
   const int rank = int(cluster.block_rank()), C = int(cluster.num_blocks());
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int row_id = int(blockIdx.x) / C, rows = int(gridDim.x) / C;
@@ -147,6 +150,7 @@ sample_typical_kernel(const float* __restrict__ x, int n, long long ldx, float t
   mx = warp_max(mx);
   if (lane == 0) S.warp_mx[warp] = mx;
   __syncthreads();
+  cluster.barrier_wait(std::move(started));    // every CTA of the cluster runs, so its shared memory exists
   if (tid < C) {
     for (int w = 0; w < kSampleWarps; ++w) mx = fmaxf(mx, S.warp_mx[w]);
     *cluster.map_shared_rank(&S.mx[rank], tid) = mx;
