@@ -180,6 +180,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) dense_tile_gemm_kernel(const 
       if (++slot == NS) { slot = 0; phase ^= 1u; }
     }
     *issued_ptr = issued;
+    if (kPair && ld.it >= nitems_all) ring_drain(empty0, slot, phase, NS, abort_flag, P.status, B200RWKV_STATUS_WAIT_EMPTY);
   } else if (warp == 1) {
     // ---------------------------------------------------------------- MMA issuer (the even CTA's, for both)
     if (rank == 0) {

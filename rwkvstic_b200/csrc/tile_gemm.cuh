@@ -231,6 +231,17 @@ __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatil
   return ok;
 }
 
+// The producer of a pair waits until every stage of its ring has been released: the MMA issuer's commits
+// arrive on the barriers of both CTAs, and a CTA must not leave before the last of them has reached it.
+// `slot`, `phase`: the stage the producer would fill next.  Stages never filled pass at once; bounded like
+// every wait, and over at once after an abort.
+__device__ __forceinline__ void ring_drain(uint32_t empty0, int slot, uint32_t phase, int stages, volatile int* abort_flag, int* status, int bit) {
+  for (int i = 0; i < stages; ++i) {
+    if (!warp_wait(empty0 + 8 * slot, phase ^ 1u, abort_flag, status, bit)) return;
+    if (++slot == stages) { slot = 0; phase ^= 1u; }
+  }
+}
+
 // Tile t of a launch -> (segment, first weight row, first activation row).  Within a matrix the order is
 // row block, weight tile, row tile of the block: the CTAs working side by side share a weight tile, and
 // all weight tiles sweep over one block of digit rows (sized by the launcher to stay in L2) before the
@@ -356,6 +367,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) tile_gemm_kernel(const __grid
         if (++slot == NS) { slot = 0; phase ^= 1u; }
       }
       *issued_ptr = issued;
+      if (kPair && ld.it >= nitems_all) ring_drain(empty0, slot, phase, NS, abort_flag, P.status, B200RWKV_STATUS_WAIT_EMPTY);
     }
   } else if (warp == 1) {
     // ---------------------------------------------------------------- MMA issuer (the even CTA's, for both)

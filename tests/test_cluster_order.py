@@ -46,3 +46,12 @@ def test_a_cluster_barrier_comes_before_the_first_access_to_another_ctas_memory(
     """A CTA of a cluster may start after its peers: its shared memory exists for them once a barrier has been met."""
     first = min(body.find(t) for t in REMOTE if t in body)
     assert any(-1 < body.find(t) < first for t in BARRIER)
+
+
+@pytest.mark.parametrize("body", [pytest.param(body, id=f"{f}:{name}") for f, name, body in kernels() if "umma_commit<kPair>(" in body])
+def test_a_producer_waits_for_the_commits_that_arrive_in_its_cta(body):
+    """tcgen05.commit with multicast arrives on a barrier in both CTAs of a pair.  A CTA that leaves while such an
+    arrival is on its way has it land in shared memory that is no longer its own, so the producer waits for the
+    release of every stage after its last copy and before the barrier in front of the exit."""
+    last_copy = max(m.start() for m in re.finditer(r"&Sg\.xmap", body))
+    assert last_copy < body.find("ring_drain(empty0") < body.rfind("cluster_sync();")
