@@ -405,10 +405,12 @@ static size_t gemm_workspace_bytes(int k_in, int nmat, int rows) {
          align256(sizeof(SegScalars) * size_t(nmat) * rows);
 }
 
-// Launch with programmatic stream serialisation: the kernel may start while its predecessor on the
-// stream is still running; every kernel launched this way calls griddepcontrol.wait before it
-// touches global memory.
-static thread_local bool g_chain_rows = true;   // set per call by forward_rows_impl / gemm_u8
+// Launches of a rows call after its first go out with programmatic stream serialisation: a kernel may start
+// while its predecessor on the stream still runs, calls griddepcontrol.wait before it touches what that or any
+// earlier kernel of the call wrote, and before the wait requests only weights and parameter vectors.  Those may
+// have been written by the work in front of the call, which nothing waits for before griddepcontrol.wait; so
+// the first launch of a call stays in plain stream order, and what follows it finds that work complete.
+static thread_local bool g_chain_launch = false;   // cleared at the start of a call, set by its first launch
 
 template <typename Kernel, typename... Args>
 static cudaError_t launch_clustered(int cluster, Kernel kernel, dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
@@ -417,7 +419,7 @@ static cudaError_t launch_clustered(int cluster, Kernel kernel, dim3 grid, dim3 
   cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = stream;
   cudaLaunchAttribute attr[2];
   int n = 0;
-  if (g_chain_rows) {
+  if (g_chain_launch) {
     attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[n++].val.programmaticStreamSerializationAllowed = 1;
   }
@@ -426,6 +428,7 @@ static cudaError_t launch_clustered(int cluster, Kernel kernel, dim3 grid, dim3 
     attr[n].val.clusterDim.x = unsigned(cluster); attr[n].val.clusterDim.y = 1; attr[n++].val.clusterDim.z = 1;
   }
   cfg.attrs = attr; cfg.numAttrs = unsigned(n);
+  g_chain_launch = true;
   return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
@@ -1641,7 +1644,7 @@ int b200rwkv_gemm_u8(int nmat, const b200rwkv_matrix* mats, const float* const* 
   P.nseg = nmat; P.K = K; P.R = rows; P.Rpad = Rpad; P.status = reinterpret_cast<int*>(wsb); P.sk_acc = sk_acc; P.sk_count = sk_count;
   const char* why = "";
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  g_chain_rows = rows <= 1024;
+  g_chain_launch = false;
   cudaError_t e = launch_rows_prep(Q, s, &why);
   if (e == cudaSuccess) e = launch_tile_gemm(P, mp, digits, s, &why);
   if (e != cudaSuccess) return fail(e == cudaErrorInvalidValue ? B200RWKV_EINVAL : B200RWKV_ECUDA, "gemm_u8: %s (%s)", why, cudaGetErrorString(e));
@@ -1677,10 +1680,11 @@ static int forward_rows_impl(const b200rwkv_model* m, const int64_t* tokens, flo
   const char* why = "";
   cudaError_t e;
 
-  // Chained at every size: the next launch's weights and parameters are requested while this one still runs
+  // Chained at every size, the first launch excepted (see g_chain_launch): the next launch's weights and parameters
+  // are requested while this one still runs
   // (decode and short prompts 10-15 % per step; bf16 3B 2 x 701 tokens 10598 -> 10154 us, uint8 3B 8 x 1024 tokens,
   // 4096 rows a call, 71868 -> 71569, within the noise).
-  g_chain_rows = true;
+  g_chain_launch = false;
   if (x_ext) ws.xa = x_ext;
   if (tokens) {
     e = launch_chained(embed_ln0_rows_kernel, dim3(R), dim3(256), 0, s, m->emb, reinterpret_cast<const long long*>(tokens), D, V,
@@ -1936,7 +1940,7 @@ int b200rwkv_dense_forward_rows_layers(const b200rwkv_dense_model* m, int layer_
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const char* why = "";
   cudaError_t e;
-  g_chain_rows = true;
+  g_chain_launch = false;
 #define B200_DR_CHECK(call, what)                                                                      \
   do {                                                                                                 \
     e = (call);                                                                                        \
