@@ -156,17 +156,6 @@ __device__ __forceinline__ float warp_max(float v) {
 
 __device__ __forceinline__ float sigmoidf_(float x) { return 1.0f / (1.0f + expf(-x)); }
 
-// n / d for operands, quotient and residual in the normal range: a reciprocal estimate and one Newton
-// correction of the quotient with its exact remainder (Markstein, 1990); within one unit of the last
-// place, without the branches and the scaling that cover the whole range of `/`.
-__device__ __forceinline__ float div_normal(float n, float d) {
-  float r;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
-  r = fmaf(fmaf(-d, r, 1.f), r, r);
-  const float q = n * r;
-  return fmaf(fmaf(-d, q, n), r, q);
-}
-
 // The state part of wkv_step.
 __device__ __forceinline__ void wkv_advance(float k, float v, float w, float& aa, float& bb, float& pp) {
   const float ww2 = pp + w;
@@ -180,15 +169,13 @@ __device__ __forceinline__ void wkv_advance(float k, float v, float w, float& aa
 
 // One WKV-4 step in the max-trick form (state aa, bb scaled by exp(-pp); decay applied when the
 // state is advanced).  Same arithmetic as the reference's agnosticRwkv.py:68-103.
-// kNormal: the division may assume ordinary magnitudes (div_normal).
-template <bool kNormal = false>
 __device__ __forceinline__ float wkv_step(float k, float v, float w, float u, float& aa, float& bb, float& pp) {
   // of each pair of exponentials exp(x - max(x, y)), exp(y - max(x, y)) one is exp(0) = 1
   const float ww = u + k;
   const float d = pp - ww, e = expf(-fabsf(d));
   const float e1 = d >= 0.f ? 1.f : e, e2 = d >= 0.f ? e : 1.f;
   const float num = e1 * aa + e2 * v, den = e1 * bb + e2;
-  const float y = kNormal ? div_normal(num, den) : num / den;
+  const float y = num / den;
   wkv_advance(k, v, w, aa, bb, pp);
   return y;
 }

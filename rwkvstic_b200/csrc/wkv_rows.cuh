@@ -113,12 +113,12 @@ __global__ void __launch_bounds__(kWkvWarpsMax * 32, 1) wkv_span_kernel(const Wk
           kk[i] = __ldcg(kp + o); vv[i] = __ldcg(vp + o); gg[i] = __ldcg(gp + o);
         }
 #pragma unroll
-        for (int i = 0; i < U; ++i) put(t + i, gg[i] * wkv_step<true>(kk[i], vv[i], wv, uv, a, b, p));
+        for (int i = 0; i < U; ++i) put(t + i, gg[i] * wkv_step(kk[i], vv[i], wv, uv, a, b, p));
       }
       for (; t < len; ++t) {
         const unsigned o = unsigned(t) * uC;
         const float k1 = __ldcg(kp + o), v1 = __ldcg(vp + o), g1 = __ldcg(gp + o);
-        put(t, g1 * wkv_step<true>(k1, v1, wv, uv, a, b, p));
+        put(t, g1 * wkv_step(k1, v1, wv, uv, a, b, p));
       }
     }
     if (len > 0 && first + len == T) { P.aa[so] = a; P.bb[so] = b; P.pp[so] = p; }
