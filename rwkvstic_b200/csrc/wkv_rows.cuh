@@ -79,7 +79,8 @@ __global__ void __launch_bounds__(kWkvWarpsMax * 32, 1) wkv_span_kernel(const Wk
     __syncthreads();
     // (a, b, p) after the steps of warps j0 .. j0 + cnt - 1
     auto advance = [&](float& a, float& b, float& p, int j0, int cnt) {
-      const float wn = wv * float(n);
+      // finite for a decay of minus infinity (a channel that forgets at once): 0 steps of it are 0, not NaN
+      const float wn = fmaxf(wv * float(n), -1e36f);
       float m = p + float(cnt) * wn;
       for (int j = 0; j < cnt; ++j) m = fmaxf(m, sp[j0 + j][lane] + float(cnt - 1 - j) * wn);
       const float e0 = expf(p + float(cnt) * wn - m);

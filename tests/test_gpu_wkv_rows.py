@@ -33,3 +33,12 @@ def test_a_state_of_zeros_with_a_first_weight_below_the_normal_range(T):
     for i in range(2):
         ck[f"blocks.{i}.att.time_first"].fill_(-88.5)
     compare(ck, lambda m, B: torch.zeros_like(m.empty_batch_state(B)), 2, T)
+
+
+@pytest.mark.parametrize("T", [2, 5, 20, 300, 700])
+def test_channels_that_forget_at_once(T):
+    """time_decay = 100 overflows to w = -exp(100) = -inf: the state after a step is that step alone."""
+    ck = synth_checkpoint(2, 128, vocab=V, seed=31)
+    for i in range(2):
+        ck[f"blocks.{i}.att.time_decay"][::7] = 100.0
+    compare(ck, lambda m, B: m.empty_batch_state(B), 2, T)
