@@ -444,7 +444,9 @@ dense_rows_prep_kernel(const __grid_constant__ DRowsPrepParams P) {
     stream_reduce<1, 0>(q, red, phase, nwarps);
     const float sd = sqrtf(q[0] / float(D) + 1e-5f);
     // n / sd by the correctly rounded reciprocal and the exact remainder of the first quotient (Markstein,
-    // 1990): the division's own result, without its range checks; a quotient by infinity stays 0
+    // 1990): the division's own result without its range checks (every mantissa of sd against 160 numerators on
+    // a CPU: no difference; fp16 1.5B 48 streams 1613 us, 1648 with the division).  Below 2^-100 the remainder of n
+    // loses bits and the quotient may be one off in its last place; a quotient by infinity stays 0.
     const float rcp = 1.0f / sd, neg = sd < INFINITY ? -sd : 0.f;
     auto quot = [&](float n) { const float q0 = n * rcp; return fmaf(fmaf(neg, q0, n), rcp, q0); };
 #pragma unroll
