@@ -160,9 +160,7 @@ sample_typical_kernel(const float* __restrict__ x, int n, long long ldx, float t
   mx = S.mx[0];
   for (int c = 1; c < C; ++c) mx = fmaxf(mx, S.mx[c]);
 
-  // ---- Z = sum e^d and sum d e^d (d = l - mx); entropy = log Z - (sum d e^d) / Z.  All terms of a sum
-  // have one sign: four are added in fp32 before they join the fp64 sum (conversions to fp64 go through
-  // a slow pipe); the rounding of those adds, 2^-24 of a term and random, vanishes beside the terms' own.
+  // ---- Z = sum e^d and sum d e^d (d = l - mx), every term in fp64; entropy = log Z - (sum d e^d) / Z
   double z = 0.0, dz = 0.0;
   auto add4 = [&](const float (&d)[4]) {
     float e[4], de[4];
@@ -171,8 +169,8 @@ sample_typical_kernel(const float* __restrict__ x, int n, long long ldx, float t
       e[j] = expf(d[j]);
       de[j] = e[j] > 0.f ? d[j] * e[j] : 0.f;
     }
-    z += double((e[0] + e[1]) + (e[2] + e[3]));
-    dz += double((de[0] + de[1]) + (de[2] + de[3]));
+    z += (double(e[0]) + double(e[1])) + (double(e[2]) + double(e[3]));
+    dz += (double(de[0]) + double(de[1])) + (double(de[2]) + double(de[3]));
   };
   int at = tid;
   for (; at + 3 * kSampleThreads < len; at += 4 * kSampleThreads) {

@@ -71,3 +71,17 @@ def test_infinite_and_equal_logits():
     tok, kept = tok.tolist(), (probs > 0).cpu()
     assert tok[0] == 31337 and tok[1] == 50276 and abs(tok[2] - 25138) <= 1 and 1000 <= tok[3] < 1100
     assert kept.sum(1).tolist()[:3] == [1, 2, 50277] and not kept[3, :1000].any() and not kept[3, 1100:].any()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [2048, 4096, 16384, 65536])
+def test_small_terms_of_the_softmax_sum_are_not_lost(n):
+    """One token in four at the maximum, the others e^-17.5 of it: together they are 7.5e-8 of Z, more than fp32
+    resolves, but each is less than half a unit of the last place of a 1.  The probability of the likely tokens is
+    1 / Z, so it shows whether Z kept them."""
+    from rwkvstic_b200 import ops
+    x = torch.full((1, n), -17.5)
+    x[0].view(-1, 512)[::4] = 0.0
+    z = np.exp(x[0].double().numpy()).sum()
+    tok, probs = ops.sample_typical(x.to(DEV), 1.0, 0.9, u=torch.tensor([0.5], device=DEV), return_probs=True)
+    assert float(probs.max()) == np.float32(1.0 / z)
