@@ -324,6 +324,7 @@ int b200rwkv_argmax(const float* x, int rows, int n, int64_t ldx, int64_t* out, 
  *   out       device int64 [rows]
  *   probs_out optional device f32 [rows][n]: the masked, tempered, unnormalised probabilities
  *   history   as b200rwkv_argmax; needs rows == 1
+ * A row's result depends on its logits and its number alone, not on the other rows of the call.
  * The reference draws with torch.multinomial, whose random stream cannot be matched; what is
  * matched is the distribution it draws from (same kept set, same weights).
  */

@@ -684,31 +684,41 @@ argmax_rows_kernel(const float* __restrict__ x, int n, long long ldx, long long*
   }
 }
 
-static cudaError_t launch_sample(const float* x, int rows, int n, long long ldx, float temp, float tau, const float* u, long long* out,
-                                 float* probs_out, long long* hist, int* hist_count, int hist_cap, cudaStream_t stream) {
+template <bool kInSmem, int kParts>
+static cudaError_t launch_sample_as(const float* x, int rows, int n, long long ldx, float temp, float tau, const float* u, long long* out,
+                                    float* probs_out, long long* hist, int* hist_count, int hist_cap, cudaStream_t stream) {
   static bool configured[64];
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
   if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
-  if (!configured[dev]) {
-    e = cudaFuncSetAttribute(sample_typical_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSampleMaxSlice * 4);
+  if (kInSmem && !configured[dev]) {
+    e = cudaFuncSetAttribute(sample_typical_kernel<kInSmem, kParts>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSampleMaxSlice * 4);
     if (e != cudaSuccess) return e;
     configured[dev] = true;
   }
-  const int c = sample_cluster(rows, n, device_sms());
-  const int slice = (n + c - 1) / c;
-  const bool in_smem = slice <= kSampleMaxSlice;
+  const unsigned c = kSampleParts / kParts;
+  const int part = sample_part(n);
   cudaLaunchConfig_t cfg;
   memset(&cfg, 0, sizeof(cfg));
-  cfg.gridDim = dim3(unsigned(rows) * unsigned(c)); cfg.blockDim = dim3(kSampleThreads); cfg.stream = stream;
-  cfg.dynamicSmemBytes = in_smem ? size_t(slice) * 4 : 0;
+  cfg.gridDim = dim3(unsigned(rows) * c); cfg.blockDim = dim3(kSampleThreads); cfg.stream = stream;
+  cfg.dynamicSmemBytes = kInSmem ? size_t(part) * kParts * 4 : 0;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = unsigned(c); attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+  attr[0].val.clusterDim.x = c; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr; cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, in_smem ? sample_typical_kernel<true> : sample_typical_kernel<false>, x, n, ldx, temp, tau, u, out,
-                            probs_out, hist, hist_count, hist_cap, slice);
+  return cudaLaunchKernelEx(&cfg, sample_typical_kernel<kInSmem, kParts>, x, n, ldx, temp, tau, u, out, probs_out, hist, hist_count, hist_cap, part);
+}
+
+static cudaError_t launch_sample(const float* x, int rows, int n, long long ldx, float temp, float tau, const float* u, long long* out,
+                                 float* probs_out, long long* hist, int* hist_count, int hist_cap, cudaStream_t stream) {
+  auto as = [&](auto launch) { return launch(x, rows, n, ldx, temp, tau, u, out, probs_out, hist, hist_count, hist_cap, stream); };
+  switch (sample_cluster(rows, n, device_sms())) {
+    case 1: return as(launch_sample_as<true, 8>);
+    case 2: return as(launch_sample_as<true, 4>);
+    case 4: return as(launch_sample_as<true, 2>);
+    default: return sample_part(n) <= kSampleMaxSlice ? as(launch_sample_as<true, 1>) : as(launch_sample_as<false, 1>);
+  }
 }
 
 // ---------------------------------------------------------------------------------------- static scratch

@@ -19,9 +19,11 @@
 // What bounds it: instruction issue and the latency of dependent passes, not bytes.  The row is read
 // from memory once, into the shared memory of its cluster (each CTA holds a slice), and the four passes
 // over it (maximum, softmax sums, histogram, draw sums with the candidates set aside) run from there.
-// Measured at n = 50277: 1 row 19 us, 74 rows 30, 148 rows 40, 256 rows 76 (two waves of clusters), against
-// 62 us for 1 row and 111 for 256 with one CTA of 1024 threads per row and eight passes through L2.  ncu
-// (256 rows): 0.57 instructions issued per clock and scheduler, the rest fixed latencies and barriers.
+// Measured at n = 50277, logits from HBM: 1 row 27 us, 37 rows 38, 74 rows 44, 148 rows 57, 256 rows 102 (two
+// waves of clusters), against 68, 72, 72, 74 and 138 with one CTA of 1024 threads per row and eight passes
+// through L2.  Of these, sums in fp64 per term (conversions go through a slow pipe) and in fixed parts cost 9 us
+// at 256 rows and 1 at 1; parts added up in the order of whatever CTAs a row got would save 5 of the 9, but
+// then the last bit of a row's sums would depend on the number of rows in the call.
 #pragma once
 
 #include <cooperative_groups.h>
@@ -35,6 +37,7 @@ namespace b200 {
 constexpr int kSampleThreads = 512;
 constexpr int kSampleWarps = kSampleThreads / 32;
 constexpr int kSampleMaxCluster = 8;
+constexpr int kSampleParts = kSampleMaxCluster;    // a row is summed in this many parts, whatever its CTAs
 constexpr int kSampleBins = 2 * kSampleThreads;    // intervals of s; the last one also takes everything beyond
 constexpr float kSampleBinsPerUnit = 64.f;         // 1/64 nat each
 constexpr int kSampleListCap = 1280;               // candidates the list holds
@@ -44,7 +47,10 @@ constexpr float kMassScale = 2147483648.0f;        // 2^31
 // Two CTAs share an SM (its 228 KB hold two slices of this many logits and the scratch), so that one
 // computes while the other waits for loads or its cluster.  Shared memory beyond that is not used.
 constexpr int kSampleMaxSlice = 25600;
-static_assert(kSampleMaxSlice <= 63 * kSampleThreads, "a thread's tokens must fit its 64-bit candidate mask");
+// consecutive tokens per thread and part (odd: no bank conflicts)
+__host__ __device__ constexpr int sample_chunk(int part) { return ((part + kSampleThreads - 1) / kSampleThreads) | 1; }
+static_assert(sample_chunk(kSampleMaxSlice) <= 64 && 2 * sample_chunk(kSampleMaxSlice / 2) <= 64 && 4 * sample_chunk(kSampleMaxSlice / 4) <= 64 &&
+                  8 * sample_chunk(kSampleMaxSlice / 8) <= 64, "a thread's tokens must fit its 64-bit candidate mask");
 
 struct TypicalRow {
   float mx;       // largest logit
@@ -74,13 +80,13 @@ struct SampleShared {
     unsigned hist[2][kSampleBins];                           // mass per interval; lane parity picks the copy
     struct { uint2 cand[kSampleListCap]; unsigned bins[256]; } list;   // (bits of s, mass) of the candidates; rank 0's is used
     unsigned radix[kSampleHists][kSampleHistStride];
+    struct { double a[kSampleParts * kSampleWarps], b[kSampleParts * kSampleWarps]; } sums;   // per part and warp
     double part[kSampleThreads];                             // draw mass per thread
   };
-  double warp_z[kSampleWarps], warp_dz[kSampleWarps];
   unsigned long long warp_sum[kSampleWarps];
   float warp_mx[kSampleWarps];
-  // one entry per CTA of the cluster, written by that CTA
-  double z[kSampleMaxCluster], dz[kSampleMaxCluster], total[kSampleMaxCluster];
+  // one entry per part of the row, or CTA of the cluster, written by the CTA that has it
+  double z[kSampleParts], dz[kSampleParts], total[kSampleParts];
   float mx[kSampleMaxCluster];
   TypicalRow row;
   unsigned long long below;     // mass in front of the interval / of the prefix
@@ -88,6 +94,8 @@ struct SampleShared {
   int bin;                      // interval of the threshold; kSampleBins: everything is kept
   int count;                    // candidates (rank 0's)
   unsigned thresh;              // bits of the threshold
+  double uniform;               // the number the draw is made with
+  int seen;                     // draws in the history before this one
 };
 
 // Sum of v over the threads before this one.
@@ -107,29 +115,63 @@ __device__ __forceinline__ unsigned long long sample_exclusive_scan(unsigned lon
   return before;
 }
 
+// Sums over a warp of N values per lane, each by the butterfly of distances 16, 8, 4, 2, 1, of which a lane follows one
+// value only: lane l returns the total of value l / (32 / N).
+template <int N>
+__device__ __forceinline__ double sample_warp_totals(double (&v)[N]) {
+  const int lane = threadIdx.x & 31;
+  int n = N;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    if (n > 1) {
+      n /= 2;
+#pragma unroll
+      for (int i = 0; i < N / 2; ++i)
+        if (i < n) {
+          const double keep = lane & o ? v[i + n] : v[i], give = lane & o ? v[i] : v[i + n];
+          v[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+        }
+    } else {
+      v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+    }
+  }
+  return v[0];
+}
+
 // logits [rows][ldx]; u: one uniform number in [0,1) per draw, read at u[row + rows * step] where
 // step = *history_count when a history is kept and 0 otherwise; out[row] = sampled id;
 // probs_out (nullable) [rows][n]: the masked, tempered, unnormalised probabilities the draw used.
-// A cluster handles a row, each of its CTAs `slice` consecutive logits.  kInSmem: the slice is held in
-// dynamic shared memory (4 * slice bytes); else (rows beyond 8 x kSampleMaxSlice logits) every pass
-// reads it from memory.
-template <bool kInSmem>
+// A cluster handles a row of kSampleParts parts of `part` consecutive logits (the last ones may be shorter or
+// empty); each of its CTAs takes kParts consecutive ones, its slice.  Sums of fp64 terms are formed
+// per part, by all threads of the CTA in the same order, and added in the order of the parts, so a row's
+// probabilities and its draw do not depend on how many CTAs it got, and with that on the rows beside it.
+// kInSmem: the slice is held in dynamic shared memory (4 bytes a logit); else (rows beyond 8 x
+// kSampleMaxSlice logits) every pass reads it from memory.
+template <bool kInSmem, int kParts>
 __global__ void __launch_bounds__(kSampleThreads, 2)
 sample_typical_kernel(const float* __restrict__ x, int n, long long ldx, float temp, float tau,
                       const float* __restrict__ u, long long* __restrict__ out, float* __restrict__ probs_out,
-                      long long* __restrict__ hist, int* __restrict__ hist_count, int hist_cap, int slice) {
+                      long long* __restrict__ hist, int* __restrict__ hist_count, int hist_cap, int part) {
   extern __shared__ float held[];
   __shared__ SampleShared S;
   namespace cg = cooperative_groups;
   const cg::cluster_group cluster = cg::this_cluster();
   auto started = cluster.barrier_arrive();     // met before the first access to another CTA's memory
-  const int rank = int(cluster.block_rank()), C = int(cluster.num_blocks());
+  const int rank = int(cluster.block_rank()), C = int(cluster.num_blocks());   // kSampleParts / kParts
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int row_id = int(blockIdx.x) / C, rows = int(gridDim.x) / C;
-  const long long first = (long long)rank * slice;
+  const long long slice = (long long)kParts * part, first = rank * slice;
   const int lo = int(first < n ? first : n), len = int(first + slice < n ? first + slice : n) - lo;
   const float* row = x + size_t(row_id) * ldx + lo;
   auto logit = [&](int i) -> float { return kInSmem ? held[i] : __ldg(row + i); };
+
+  if (tid == 0) {
+    // u holds rows * history_capacity numbers when a history is kept: replays beyond the capacity reuse the last one
+    int step = (hist && hist_count) ? *hist_count : 0;
+    S.seen = step;
+    if (step >= hist_cap && hist_cap > 0) step = hist_cap - 1;
+    S.uniform = double(u[row_id + size_t(rows) * step]);
+  }
 
   // ---- the slice into shared memory, and the largest logit
   float mx = -INFINITY;
@@ -155,52 +197,59 @@ sample_typical_kernel(const float* __restrict__ x, int n, long long ldx, float t
     for (int w = 0; w < kSampleWarps; ++w) mx = fmaxf(mx, S.warp_mx[w]);
     *cluster.map_shared_rank(&S.mx[rank], tid) = mx;
   }
-  for (int i = tid; i < 2 * kSampleBins; i += kSampleThreads) (&S.hist[0][0])[i] = 0u;
   cluster.sync();
   mx = S.mx[0];
   for (int c = 1; c < C; ++c) mx = fmaxf(mx, S.mx[c]);
 
   // ---- Z = sum e^d and sum d e^d (d = l - mx), every term in fp64; entropy = log Z - (sum d e^d) / Z
-  double z = 0.0, dz = 0.0;
-  auto add4 = [&](const float (&d)[4]) {
-    float e[4], de[4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      e[j] = expf(d[j]);
-      de[j] = e[j] > 0.f ? d[j] * e[j] : 0.f;
-    }
-    z += (double(e[0]) + double(e[1])) + (double(e[2]) + double(e[3]));
-    dz += (double(de[0]) + double(de[1])) + (double(de[2]) + double(de[3]));
+  // sums of the parts, over the warps in their order (part_total); the lanes that hold a part's sum of their warp write it
+  constexpr int kPartLanes = 32 / kParts;
+  const int lane_part = lane / kPartLanes;
+  const bool lane_writes = lane % kPartLanes == 0;
+  auto part_total = [&](const double* w, int p) {
+    double t = 0.0;
+    for (int i = 0; i < kSampleWarps; ++i) t += w[p * kSampleWarps + i];
+    return t;
   };
-  int at = tid;
-  for (; at + 3 * kSampleThreads < len; at += 4 * kSampleThreads) {
-    float d[4];
+  double zs[kParts], dzs[kParts];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) d[j] = logit(at + j * kSampleThreads) - mx;
-    add4(d);
-  }
-  for (; at < len; at += kSampleThreads) {
-    const float d = logit(at) - mx, e = expf(d);
-    z += double(e);
-    if (e > 0.f) dz += double(d * e);
-  }
+  for (int p = 0; p < kParts; ++p) {
+    const int end = min(len, (p + 1) * part);
+    double z = 0.0, dz = 0.0;
+    int at = p * part + tid;
+    for (; at + 3 * kSampleThreads < end; at += 4 * kSampleThreads) {
+      float e[4], de[4];
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    z += __shfl_xor_sync(0xffffffffu, z, o);
-    dz += __shfl_xor_sync(0xffffffffu, dz, o);
+      for (int j = 0; j < 4; ++j) {
+        const float d = logit(at + j * kSampleThreads) - mx;
+        e[j] = expf(d);
+        de[j] = e[j] > 0.f ? d * e[j] : 0.f;
+      }
+      z += (double(e[0]) + double(e[1])) + (double(e[2]) + double(e[3]));
+      dz += (double(de[0]) + double(de[1])) + (double(de[2]) + double(de[3]));
+    }
+    for (; at < end; at += kSampleThreads) {
+      const float d = logit(at) - mx, e = expf(d);
+      z += double(e);
+      if (e > 0.f) dz += double(d * e);
+    }
+    zs[p] = z; dzs[p] = dz;
   }
-  if (lane == 0) { S.warp_z[warp] = z; S.warp_dz[warp] = dz; }
+  {
+    const double z = sample_warp_totals(zs), dz = sample_warp_totals(dzs);
+    if (lane_writes) { S.sums.a[lane_part * kSampleWarps + warp] = z; S.sums.b[lane_part * kSampleWarps + warp] = dz; }
+  }
   __syncthreads();
-  if (tid < C) {
-    z = 0.0; dz = 0.0;
-    for (int w = 0; w < kSampleWarps; ++w) { z += S.warp_z[w]; dz += S.warp_dz[w]; }
-    *cluster.map_shared_rank(&S.z[rank], tid) = z;
-    *cluster.map_shared_rank(&S.dz[rank], tid) = dz;
+  if (tid < kSampleParts) {                  // thread: a part of this CTA and a CTA to tell
+    const int p = tid / C, to = tid - p * C;
+    *cluster.map_shared_rank(&S.z[rank * kParts + p], to) = part_total(S.sums.a, p);
+    *cluster.map_shared_rank(&S.dz[rank * kParts + p], to) = part_total(S.sums.b, p);
   }
   cluster.sync();
+  for (int i = tid; i < 2 * kSampleBins; i += kSampleThreads) (&S.hist[0][0])[i] = 0u;
   if (tid == 0) {
-    z = 0.0; dz = 0.0;
-    for (int c = 0; c < C; ++c) { z += S.z[c]; dz += S.dz[c]; }     // the same order in every CTA
+    double z = 0.0, dz = 0.0;
+    for (int p = 0; p < kSampleParts; ++p) { z += S.z[p]; dz += S.dz[p]; }
     const double lz = log(z);
     S.row.mx = mx;
     S.row.inv_z = float(1.0 / z);
@@ -258,48 +307,62 @@ sample_typical_kernel(const float* __restrict__ x, int n, long long ldx, float t
   const int bin = S.bin;
 
   // ---- draw sums, q_i = keep_i ? p_i^(1/temp) : 0 in index order.  A thread owns `chunk` consecutive
-  // tokens (odd: no bank conflicts).  Below the interval a token is kept; inside it is a candidate, noted
-  // in the thread's mask and, with its mass, in rank 0's list.
+  // tokens of every part.  Below the interval a token is kept; inside it is a candidate, noted in the
+  // thread's mask and, with its mass, in rank 0's list.
   const float inv_temp = 1.0f / temp;
   const bool tempered = temp != 1.0f;
   auto temper = [&](float q) { return tempered && q > 0.f ? powf(q, inv_temp) : q; };
-  const int chunk = ((slice + kSampleThreads - 1) / kSampleThreads) | 1;
-  const int i0 = min((long long)tid * chunk, (long long)len), i1 = min((long long)i0 + chunk, (long long)len);
-  double mine = 0.0;
-  unsigned long long mask = 0ull;
+  const int chunk = sample_chunk(part);
+  auto part_begin = [&](int p) { return int(min((long long)p * part + (long long)tid * chunk, (long long)min(len, (p + 1) * part))); };
+  auto part_end = [&](int p) { return int(min((long long)p * part + (long long)(tid + 1) * chunk, (long long)min(len, (p + 1) * part))); };
+  double mine[kParts];                       // per part
+  unsigned long long mask = 0ull;            // bit p * chunk + j: token j of the thread's in part p is a candidate
   {
     uint2* cand0 = cluster.map_shared_rank(&S.list.cand[0], 0);
     int* count0 = cluster.map_shared_rank(&S.count, 0);
-    auto candidate = [&](int i, float l, float s) {
-      if (kInSmem) mask |= 1ull << (i - i0);
+    auto candidate = [&](int bit, float l, float s) {
+      if (kInSmem) mask |= 1ull << bit;
       const unsigned m = typical_mass(typical_prob(l, r));
       if (m) {
         const int slot = atomicAdd(count0, 1);
         if (slot < kSampleListCap) cand0[slot] = make_uint2(__float_as_uint(s), m);
       }
     };
-    // four tokens at a time without branches but for the rare candidates: some lane keeps each of them
-    for (int i = i0; i < i1; i += 4) {
-      float l[4], s[4], q[4];
-      int b[4];
-      bool any = false;
+#pragma unroll 1
+    for (int p = 0; p < kParts; ++p) {
+      const int i0 = part_begin(p), i1 = part_end(p);
+      double sum = 0.0;
+      int i = i0;
+      // four tokens at a time without branches but for the rare candidates: some lane keeps each of them
+      for (; i + 3 < i1; i += 4) {
+        float l[4], s[4], q[4];
+        int b[4];
+        bool any = false;
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        l[j] = i + j < i1 ? logit(i + j) : -INFINITY;
-        s[j] = typical_shift(l[j], r);
-        b[j] = i + j < i1 ? typical_bin(s[j]) : 2 * kSampleBins;
-        q[j] = b[j] < bin ? typical_prob(l[j], r) : 0.f;
-        any = any || b[j] == bin;
-      }
-      if (kInSmem) {
+        for (int j = 0; j < 4; ++j) {
+          l[j] = logit(i + j);
+          s[j] = typical_shift(l[j], r);
+          b[j] = typical_bin(s[j]);
+          q[j] = b[j] < bin ? typical_prob(l[j], r) : 0.f;
+          any = any || b[j] == bin;
+        }
+        if (kInSmem) {
 #pragma unroll
-        for (int j = 0; j < 4; ++j) mine += double(temper(q[j]));
-      }
-      if (any) {
+          for (int j = 0; j < 4; ++j) sum += double(temper(q[j]));
+        }
+        if (any) {
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
-          if (b[j] == bin) candidate(i + j, l[j], s[j]);
+          for (int j = 0; j < 4; ++j)
+            if (b[j] == bin) candidate(p * chunk + i + j - i0, l[j], s[j]);
+        }
       }
+      for (; i < i1; ++i) {
+        const float l = logit(i), s = typical_shift(l, r);
+        const int b = typical_bin(s);
+        if (kInSmem && b < bin) sum += double(temper(typical_prob(l, r)));
+        if (b == bin) candidate(p * chunk + i - i0, l, s);
+      }
+      mine[p] = sum;
     }
   }
   cluster.sync();
@@ -362,16 +425,54 @@ sample_typical_kernel(const float* __restrict__ x, int n, long long ldx, float t
     const float p = typical_prob(l, r);
     return temper((keep_all || typical_shift(l, r) <= thresh) ? p : 0.f);
   };
-  if (kInSmem) {
-    for (; mask; mask &= mask - 1) mine += double(weight(logit(i0 + __ffsll(mask) - 1)));
-  } else {
-    for (int i = i0; i < i1; ++i) mine += double(weight(logit(i)));
-  }
   if (probs_out)
     for (int i = tid; i < len; i += kSampleThreads) probs_out[size_t(row_id) * n + lo + i] = weight(logit(i));
 
-  // ---- the draw: inverse CDF over the CTAs of the cluster, the threads of one CTA, the tokens of one thread
-  S.part[tid] = mine;
+  // ---- the draw: inverse CDF over the parts, the threads of one part, the tokens of one thread
+#pragma unroll
+  for (int p = 0; p < kParts; ++p) {
+    double sum = mine[p];
+    const int i0 = part_begin(p);
+    if (kInSmem) {
+      for (unsigned long long some = mask >> (p * chunk) & ((1ull << chunk) - 1); some; some &= some - 1)
+        sum += double(weight(logit(i0 + __ffsll(some) - 1)));
+    } else {
+      const int i1 = part_end(p);
+      for (int i = i0; i < i1; ++i) sum += double(weight(logit(i)));
+    }
+    mine[p] = sum;
+  }
+  {
+    double v[kParts];
+#pragma unroll
+    for (int p = 0; p < kParts; ++p) v[p] = mine[p];
+    const double sum = sample_warp_totals(v);
+    if (lane_writes) S.sums.a[lane_part * kSampleWarps + warp] = sum;
+  }
+  __syncthreads();
+  if (tid < kSampleParts) {
+    const int p = tid / C, to = tid - p * C;
+    *cluster.map_shared_rank(&S.total[rank * kParts + p], to) = part_total(S.sums.a, p);
+  }
+  cluster.sync();               // the last access to another CTA's memory
+  double total = 0.0;
+  for (int p = 0; p < kSampleParts; ++p) total += S.total[p];
+  const double target = S.uniform * total;
+  int owner_part = -1, last_part = 0;
+  double base = 0.0, before = 0.0, last_before = 0.0;      // mass in front of the owner's part
+  for (int p = 0; p < kSampleParts; ++p) {
+    const double v = S.total[p];
+    if (v > 0.0) {
+      last_part = p; last_before = before;
+      if (owner_part < 0 && before + v >= target) { owner_part = p; base = before; }
+    }
+    before += v;
+  }
+  // rounding can leave the target past the end: the last that holds any mass
+  if (owner_part < 0) { owner_part = last_part; base = last_before; }
+  if (owner_part / kParts != rank) return;
+  const int mine_part = owner_part - rank * kParts;
+  S.part[tid] = mine[mine_part];
   __syncthreads();
   if (warp == 0) {
     // lane l owns the partial sums of threads [16 l, 16 l + 16)
@@ -384,31 +485,12 @@ sample_typical_kernel(const float* __restrict__ x, int n, long long ldx, float t
       const double t = __shfl_up_sync(0xffffffffu, inc, o);
       if (lane >= o) inc += t;
     }
-    const double cta_total = __shfl_sync(0xffffffffu, inc, 31);
-    if (lane < C) *cluster.map_shared_rank(&S.total[rank], lane) = cta_total;
-    // u holds rows * history_capacity numbers when a history is kept: replays beyond the capacity reuse the last one
-    int step = (hist && hist_count) ? *hist_count : 0;
-    const int seen = step;
-    if (step >= hist_cap && hist_cap > 0) step = hist_cap - 1;
-    const double uniform = double(u[row_id + size_t(rows) * step]);
-    cluster.sync();             // the last access to another CTA's memory
-    double total = 0.0, base = 0.0;
-    for (int c = 0; c < C; ++c) { if (c == rank) base = total; total += S.total[c]; }
-    const double target = uniform * total;
-    int owner_cta = -1, last_cta = 0;
-    double run = 0.0;
-    for (int c = 0; c < C; ++c) {
-      run += S.total[c];
-      if (S.total[c] > 0.0) { last_cta = c; if (owner_cta < 0 && run >= target) owner_cta = c; }
-    }
-    if (owner_cta < 0) owner_cta = last_cta;   // rounding can leave the target past the end: the last that holds any mass
-    if (rank != owner_cta) return;
     inc += base;
     const unsigned hit = __ballot_sync(0xffffffffu, loc > 0.0 && inc >= target);
     const unsigned nonzero = __ballot_sync(0xffffffffu, loc > 0.0);
     const int owner = hit ? __ffs(hit) - 1 : (nonzero ? 31 - __clz(nonzero) : 0);
     // the thread of that group whose tokens hold the target (the same search, in the owner's order)
-    run = __shfl_sync(0xffffffffu, inc - loc, owner);
+    double run = __shfl_sync(0xffffffffu, inc - loc, owner);
     int c = -1, last = owner * kPer;
     double run_last = run;
     for (int k = 0; k < kPer; ++k) {
@@ -422,7 +504,8 @@ sample_typical_kernel(const float* __restrict__ x, int n, long long ldx, float t
     if (c < 0) c = last;
     run = run_last;
     // its tokens, 32 at a time
-    const int j0 = min((long long)c * chunk, (long long)len), j1 = min((long long)j0 + chunk, (long long)len);
+    const int end = min(len, (mine_part + 1) * part);
+    const int j0 = int(min((long long)mine_part * part + (long long)c * chunk, (long long)end)), j1 = min(j0 + chunk, end);
     int pick = -1, kept = j0;
     for (int b = j0; b < j1 && pick < 0; b += 32) {
       const float q = b + lane < j1 ? weight(logit(b + lane)) : 0.f;
@@ -442,21 +525,21 @@ sample_typical_kernel(const float* __restrict__ x, int n, long long ldx, float t
       const long long id = (long long)lo + (pick < 0 ? kept : pick);
       out[row_id] = id;
       if (hist && hist_count && row_id == 0) {
-        if (seen < hist_cap) hist[seen] = id;
-        *hist_count = seen + 1;
+        if (S.seen < hist_cap) hist[S.seen] = id;
+        *hist_count = S.seen + 1;      // every CTA has read it: it did before the first cluster barrier
       }
     }
-  } else {
-    cluster.sync();
   }
 }
 
+inline int sample_part(int n) { return n / kSampleParts + (n % kSampleParts != 0); }
+
 // CTAs per row: the fewest whose slices fit two to an SM, and more while the launch still leaves SMs
-// without a CTA and a slice has four tokens or more per thread (50277 logits: 19 us for 1 row with 8 CTAs,
-// 27 for 37 rows with 4, 30 for 74 rows with 2).
+// without a CTA and a slice has four tokens or more per thread (50277 logits: 27 us for 1 row with 8 CTAs,
+// 38 for 37 rows with 4, 44 for 74 rows with 2).
 inline int sample_cluster(int rows, int n, int sms) {
   int c = 1;
-  while (c < kSampleMaxCluster && (n + c - 1) / c > kSampleMaxSlice) c *= 2;
+  while (c < kSampleMaxCluster && sample_part(n) > c * (kSampleMaxSlice / kSampleParts)) c *= 2;
   while (c < kSampleMaxCluster && (long long)rows * 2 * c <= sms && n / (2 * c) >= 4 * kSampleThreads) c *= 2;
   return c;
 }

@@ -85,3 +85,23 @@ def test_small_terms_of_the_softmax_sum_are_not_lost(n):
     z = np.exp(x[0].double().numpy()).sum()
     tok, probs = ops.sample_typical(x.to(DEV), 1.0, 0.9, u=torch.tensor([0.5], device=DEV), return_probs=True)
     assert float(probs.max()) == np.float32(1.0 / z)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [24576, 50277, 31])
+def test_a_row_gives_the_same_alone_and_beside_others(n):
+    """A call of few rows gives a row more CTAs than a call of many; its probabilities and its draw are the same bits.
+    The last row has one token in four at the maximum and the rest e^-17.5 of it: sums that depend on how the row is
+    cut show there."""
+    from rwkvstic_b200 import ops
+    g = torch.Generator(device=DEV).manual_seed(n)
+    x = torch.randn(300, n, generator=g, device=DEV) * 2.0
+    x[-1] = torch.where(torch.arange(n, device=DEV) // 512 % 4 == 0, 0.0, -17.5)
+    u = torch.rand(300, generator=g, device=DEV)
+    for temp, tau in [(1.0, 0.8), (0.7, 0.95)]:
+        tok, probs = ops.sample_typical(x, temp, tau, u=u, return_probs=True)
+        for rows in (1, 7, 30, 75):                  # eight, four, two CTAs a row at 50277 tokens
+            for first in (0, 111, 300 - rows):
+                at = slice(first, first + rows)
+                t, p = ops.sample_typical(x[at].contiguous(), temp, tau, u=u[at].contiguous(), return_probs=True)
+                assert torch.equal(p, probs[at]) and torch.equal(t, tok[at])
