@@ -251,14 +251,24 @@ size_t b200rwkv_gemm_workspace_bytes(int k_in, int nmat, int rows);
  * exact integer dot products, the same affine terms), so a row's result does not depend on
  * which of the two entry points computed it beyond the fp32 summation order of sum_k x*my.
  * Two launches: a row-wise preparation kernel, then a tcgen05 (kind::i8) tensor-core kernel with
- * TMA-fed operands and TMEM accumulators: persistent CTAs over tiles of 128 or 256 outputs x
- * 16..80 rows, the shape picked per launch.  rows <= 65535.
+ * TMA-fed operands and TMEM accumulators: persistent CTAs (128 outputs x
+ * 16..80 rows a tile) or pairs of CTAs (256 x 32..160), picked per launch.  rows <= 65535.
  * `workspace`: b200rwkv_gemm_workspace_bytes(k_in, nmat, rows), 256-byte aligned, ZERO-FILLED once
  * before its first use (first int = status word; it also holds the integer scratch in which launches
  * with few rows combine their K slices, which every launch leaves zero again).
  */
 int b200rwkv_gemm_u8(int nmat, const b200rwkv_matrix* mats, const float* const* x, float* const* y, int rows,
                      void* workspace, size_t workspace_bytes, void* stream);
+
+/*
+ * Host-only introspection of the tile that a tensor-core launch takes: elem_bytes 1 for uint8 matrices
+ * (b200rwkv_gemm_u8, b200rwkv_forward_rows), 2 for bf16 / fp16 ones (b200rwkv_dense_forward_rows); nmat
+ * matrices of n_out[i] outputs and k_in inputs, `rows` activation rows, a GPU with num_sms SMs.  Fills
+ * out[0..5] = {CTA pairs (0 or 1), activation rows one CTA holds of a tile, K slices per tile, 128-byte
+ * chunks of K per ring stage, ring stages, accumulator buffers}.  No counterpart in the reference; used by
+ * tests.
+ */
+int b200rwkv_gemm_plan(int elem_bytes, int nmat, int k_in, const int32_t* n_out, int rows, int num_sms, int64_t* out);
 
 /* Bytes of device scratch b200rwkv_forward_rows needs (0 if streams * tokens_per_stream > 65535);
  * zero-fill it once before its first use (status word and K-slice scratch, see b200rwkv_gemm_u8). */

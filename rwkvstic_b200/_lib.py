@@ -20,7 +20,7 @@ EXPORTS = (
     "b200rwkv_version", "b200rwkv_last_error", "b200rwkv_gemv_u8", "b200rwkv_wkv_scan", "b200rwkv_gemv_plan",
     "b200rwkv_gemv_u8_traced", "b200rwkv_gemv_workspace_bytes", "b200rwkv_gemv_u8_static",
     "b200rwkv_decode_workspace_bytes", "b200rwkv_decode_step", "b200rwkv_decode_step_traced", "b200rwkv_decode_step_stage",
-    "b200rwkv_gemm_workspace_bytes", "b200rwkv_gemm_u8", "b200rwkv_rows_workspace_bytes", "b200rwkv_forward_rows", "b200rwkv_forward_rows_stage", "b200rwkv_argmax",
+    "b200rwkv_gemm_plan", "b200rwkv_gemm_workspace_bytes", "b200rwkv_gemm_u8", "b200rwkv_rows_workspace_bytes", "b200rwkv_forward_rows", "b200rwkv_forward_rows_stage", "b200rwkv_argmax",
     "b200rwkv_sample_typical", "b200rwkv_gemv_dense",
     "b200rwkv_dense_workspace_bytes", "b200rwkv_dense_step", "b200rwkv_dense_rows_workspace_bytes", "b200rwkv_dense_forward_rows",
     "b200rwkv_dense_step_layers", "b200rwkv_dense_forward_rows_layers", "b200rwkv_wait_selftest", "b200rwkv_debug_expire_waits",
@@ -116,6 +116,8 @@ def lib() -> C.CDLL:
                                                   C.c_void_p, C.POINTER(C.c_int32), C.c_void_p, C.c_void_p]
     L.b200rwkv_step_geometry.restype = C.c_int
     L.b200rwkv_step_geometry.argtypes = [C.POINTER(Model), C.c_int, C.POINTER(C.c_int64)]
+    L.b200rwkv_gemm_plan.restype = C.c_int
+    L.b200rwkv_gemm_plan.argtypes = [C.c_int, C.c_int, C.c_int, C.POINTER(C.c_int32), C.c_int, C.c_int, C.POINTER(C.c_int64)]
     L.b200rwkv_gemm_workspace_bytes.restype = C.c_size_t
     L.b200rwkv_gemm_workspace_bytes.argtypes = [C.c_int, C.c_int, C.c_int]
     L.b200rwkv_gemm_u8.restype = C.c_int
@@ -180,3 +182,12 @@ def gemv_plan(k_in: int, nmat: int, max_n_out: int, num_sms: int = 148) -> dict:
     out = (C.c_int64 * 10)()
     check(lib().b200rwkv_gemv_plan(k_in, nmat, max_n_out, num_sms, out))
     return dict(zip(PLAN_FIELDS, [int(v) for v in out]))
+
+
+GEMM_PLAN_FIELDS = ("pair", "rows", "slices", "chunks", "stages", "buffers")
+
+
+def gemm_plan(elem_bytes: int, k_in: int, n_out, rows: int, num_sms: int = 148) -> dict:
+    out = (C.c_int64 * 6)()
+    check(lib().b200rwkv_gemm_plan(elem_bytes, len(n_out), k_in, (C.c_int32 * len(n_out))(*n_out), rows, num_sms, out))
+    return dict(zip(GEMM_PLAN_FIELDS, [int(v) for v in out]))

@@ -548,9 +548,9 @@ static cudaError_t launch_rows_prep(const RowsPrepParams& P_in, cudaStream_t str
 }
 
 // Encodes the tensor maps of P (weights and digit rows) for one tile shape and launches the tile GEMM.
-// digits: [nseg][3][Rpad][K].  kc = 0: chunks per stage by gemm_chunks_per_stage.
+// digits: [nseg][3][Rpad][K].
 static cudaError_t launch_tile_gemm_as(GemmParams& P, const b200rwkv_matrix* const* mats, const signed char* digits, bool pair, int Rt,
-                                       int ksplit, int kc, cudaStream_t stream, const char** why) {
+                                       int ksplit, cudaStream_t stream, const char** why) {
   static bool configured[64];
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
@@ -564,9 +564,9 @@ static cudaError_t launch_tile_gemm_as(GemmParams& P, const b200rwkv_matrix* con
   }
   P.pair = pair ? 1 : 0; P.Rt = Rt; P.ksplit = ksplit;
   const int weight_rows = pair ? 2 * kGemmM : kGemmM, rows_tile = pair ? 2 * Rt : Rt;
-  P.dbuf = kDigits * rows_tile <= kGemmAcc1Col ? 1 : 0;
+  P.dbuf = gemm_double_buffered(pair, Rt) ? 1 : 0;
   const int chunk = (kGemmM + kDigits * Rt) * 128, nk = P.K / 128 / ksplit;
-  P.kc = kc > 0 ? kc : gemm_chunks_per_stage(chunk, nk, pair);
+  P.kc = gemm_chunks_per_stage(chunk, nk, pair);
   P.stage_bytes = P.kc * chunk;
   P.stages = std::min(kGemmRingBytes / P.stage_bytes, kGemmMaxStages);
   for (int s = 0; s < P.nseg; ++s) {
@@ -599,9 +599,9 @@ static cudaError_t launch_tile_gemm_as(GemmParams& P, const b200rwkv_matrix* con
 // core), which is why a pair, whose CTAs each hold half of the digit rows, needs less per row.  A tile
 // whose accumulator has no second buffer waits 3.6 us for its epilogue; a K slice pays 3 us for its
 // atomics and ticket.
-static void gemm_pick_tile(const GemmParams& P, int* pair, int* Rt, int* ksplit) {
+static void gemm_pick_tile(const GemmParams& P, long long sms, int* pair, int* Rt, int* ksplit) {
   static const double step_single[5] = {0.16, 0.215, 0.26, 0.32, 0.345}, step_pair[5] = {0.18, 0.25, 0.40, 0.45, 0.555};   // Rt = 16, 32, .. 80
-  const long long sms = device_sms() > 1 ? device_sms() : 2;
+  sms = sms > 1 ? sms : 2;
   const int nk = P.K / 128;
   double best = 0.0;
   for (int pr = 0; pr <= 1; ++pr) {
@@ -611,7 +611,7 @@ static void gemm_pick_tile(const GemmParams& P, int* pair, int* Rt, int* ksplit)
       const long long row_tiles = (P.R + rows - 1) / rows;
       long long tiles = 0;
       for (int s = 0; s < P.nseg; ++s) tiles += row_tiles * ((P.seg[s].N + wrows - 1) / wrows);
-      const bool dbuf = kDigits * rows <= kGemmAcc1Col;
+      const bool dbuf = gemm_double_buffered(pr != 0, rt);
       for (int ks = 1; ks <= 8; ks *= 2) {
         // K slices: only where the scratch exists and fits, and where they create CTAs the launch lacks
         if (ks > 1 && (!P.sk_acc || pr || rt > kSplitMaxRt || tiles > kSplitMaxTiles || nk % ks != 0 || nk / ks < 4 ||
@@ -630,9 +630,10 @@ static void gemm_pick_tile(const GemmParams& P, int* pair, int* Rt, int* ksplit)
 static cudaError_t launch_tile_gemm(GemmParams& P, const b200rwkv_matrix* const* mats, const signed char* digits,
                                     cudaStream_t stream, const char** why) {
   int pair = 0, Rt = 16, ksplit = 1;
-  gemm_pick_tile(P, &pair, &Rt, &ksplit);
-  return launch_tile_gemm_as(P, mats, digits, pair != 0, Rt, ksplit, 0, stream, why);
+  gemm_pick_tile(P, device_sms(), &pair, &Rt, &ksplit);
+  return launch_tile_gemm_as(P, mats, digits, pair != 0, Rt, ksplit, stream, why);
 }
+
 static void fill_gemm_seg(GemmSeg& s, const b200rwkv_matrix& m, const SegScalars* scal, float* out, long long ldo) {
   memset(&s, 0, sizeof(s));
   s.rx = m.rx; s.mx = m.mx; s.half = m.half; s.N = m.n_out; s.act = ACT_NONE;
@@ -1044,7 +1045,7 @@ static DenseRowsWorkspace dense_carve_rows(const b200rwkv_dense_model* m, int B,
 // Encodes the tensor maps for one tile shape and launches.  w[s]: [N_s][K] of the 16-bit type; x[s]:
 // [rows_alloc][K] of the same type.
 static cudaError_t launch_dense_gemm_as(DGemmParams& P, const void* const* w, const unsigned short* const* x, int K, int rows_alloc,
-                                        bool pair, int Rt, int ksplit, int kc, cudaStream_t stream, const char** why) {
+                                        bool pair, int Rt, int ksplit, cudaStream_t stream, const char** why) {
   static bool configured[64];
   *why = "dense_tile_gemm launch failed";
   int dev = 0;
@@ -1059,7 +1060,7 @@ static cudaError_t launch_dense_gemm_as(DGemmParams& P, const void* const* w, co
   P.ksteps = K * 2 / 128;
   P.pair = pair ? 1 : 0; P.Rt = Rt; P.ksplit = ksplit;
   const int weight_rows = pair ? 256 : 128, rows_tile = pair ? 2 * Rt : Rt, chunk = (128 + Rt) * 128;
-  P.kc = kc > 0 ? kc : gemm_chunks_per_stage(chunk, P.ksteps / ksplit, pair);
+  P.kc = gemm_chunks_per_stage(chunk, P.ksteps / ksplit, pair);
   P.stage_bytes = P.kc * chunk;
   P.stages = std::min(kDgRingBytes / P.stage_bytes, kDgMaxStages);
   P.row_tiles = (P.R + rows_tile - 1) / rows_tile;
@@ -1089,8 +1090,8 @@ static double dense_gemm_step_us(bool pair, int Rt) {
   return pair ? (two ? 0.125 + 0.0012 * Rt : 0.16 + 0.00105 * Rt) : (two ? 0.14 + 0.00085 * Rt : 0.15 + 0.0009 * Rt);
 }
 
-static bool dense_gemm_pick_tile(const DGemmParams& P, int ksteps, int* pair, int* Rt, int* ksplit) {
-  const int sms = device_sms() > 1 ? device_sms() : 2;
+static bool dense_gemm_pick_tile(const DGemmParams& P, int ksteps, int sms, int* pair, int* Rt, int* ksplit) {
+  sms = sms > 1 ? sms : 2;
   double best = 0.0;
   for (int pr = 0; pr <= 1; ++pr) {
     const int unit = pr ? 32 : 16, most = pr ? 2 * kDgRowsPair : kDgRowsSingle;
@@ -1117,8 +1118,8 @@ static bool dense_gemm_pick_tile(const DGemmParams& P, int ksteps, int* pair, in
 static cudaError_t launch_dense_gemm(DGemmParams& P, const void* const* w, const unsigned short* const* x, int K, int rows_alloc,
                                      cudaStream_t stream, const char** why) {
   int pair = 0, Rt = 16, ksplit = 1;
-  if (!dense_gemm_pick_tile(P, K * 2 / 128, &pair, &Rt, &ksplit)) { *why = "no tile fits"; return cudaErrorInvalidValue; }
-  return launch_dense_gemm_as(P, w, x, K, rows_alloc, pair != 0, Rt, ksplit, 0, stream, why);
+  if (!dense_gemm_pick_tile(P, K * 2 / 128, device_sms(), &pair, &Rt, &ksplit)) { *why = "no tile fits"; return cudaErrorInvalidValue; }
+  return launch_dense_gemm_as(P, w, x, K, rows_alloc, pair != 0, Rt, ksplit, stream, why);
 }
 
 template <int G, int NT_MAX, int MIN_CTAS>
@@ -1611,6 +1612,37 @@ int b200rwkv_decode_step_persistent(const b200rwkv_model* m, void* plan, size_t 
   cfg.attrs = attr; cfg.numAttrs = 1;
   e = cudaLaunchKernelEx(&cfg, decode_step_kernel, P);
   if (e != cudaSuccess) return fail(B200RWKV_ECUDA, "decode_step_persistent: launch: %s", cudaGetErrorString(e));
+  return B200RWKV_OK;
+}
+
+int b200rwkv_gemm_plan(int elem_bytes, int nmat, int k_in, const int32_t* n_out, int rows, int num_sms, int64_t* out) {
+  if ((elem_bytes != 1 && elem_bytes != 2) || nmat < 1 || nmat > kMaxSeg || k_in < 128 || (size_t(k_in) * elem_bytes) % 128 != 0 || !n_out || rows < 1 ||
+      rows > 65535 || num_sms < 2 || !out)
+    return fail(B200RWKV_EINVAL, "gemm_plan: unsupported shape k_in=%d nmat=%d rows=%d sms=%d", k_in, nmat, rows, num_sms);
+  int pair = 0, Rt = 16, ksplit = 1, chunk;
+  bool dbuf = true;
+  const int nk = k_in * elem_bytes / 128;
+  if (elem_bytes == 1) {
+    GemmParams P;
+    memset(&P, 0, sizeof(P));
+    int scratch;
+    P.nseg = nmat; P.K = k_in; P.R = rows; P.sk_acc = &scratch;
+    for (int i = 0; i < nmat; ++i) P.seg[i].N = n_out[i];
+    gemm_pick_tile(P, num_sms, &pair, &Rt, &ksplit);
+    chunk = (kGemmM + kDigits * Rt) * 128;
+    dbuf = gemm_double_buffered(pair != 0, Rt);
+  } else {
+    DGemmParams P;
+    memset(&P, 0, sizeof(P));
+    float scratch;
+    P.nseg = nmat; P.R = rows; P.sk_part = rows <= kDgSplitMaxRows ? &scratch : nullptr;
+    for (int i = 0; i < nmat; ++i) P.seg[i].N = n_out[i];
+    if (!dense_gemm_pick_tile(P, nk, num_sms, &pair, &Rt, &ksplit)) return fail(B200RWKV_EINVAL, "gemm_plan: no tile fits");
+    chunk = (128 + Rt) * 128;
+  }
+  const int kc = gemm_chunks_per_stage(chunk, nk / ksplit, pair != 0);
+  const int64_t v[6] = {pair, Rt, ksplit, kc, std::min(kGemmRingBytes / (kc * chunk), kGemmMaxStages), dbuf ? 2 : 1};
+  for (int i = 0; i < 6; ++i) out[i] = v[i];
   return B200RWKV_OK;
 }
 

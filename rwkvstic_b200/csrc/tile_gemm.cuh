@@ -48,18 +48,18 @@ constexpr int kGemmAcc1Col = 256;                        // first column of the 
 constexpr int kGemmEpiWarps = 16;                        // four per TMEM lane quadrant
 constexpr int kGemmThreads = 128 + kGemmEpiWarps * 32;   // warp 0 TMA, 1 MMA, 2 TMEM allocation, 4.. epilogue
 constexpr int kGemmChunk = 8;                            // activation rows an epilogue warp handles per TMEM read
-// 8-row chunks of both 128-row sub-tiles that one epilogue warp takes at most (every fourth of its lane quadrant's)
+// 8-row chunks of a tile (of a pair: 160 rows) that one epilogue warp takes at most, every fourth of its lane quadrant's
 constexpr int kGemmItemsPerWarp = (2 * (kGemmRowsMax / kGemmChunk) + kGemmEpiWarps / 4 - 1) / (kGemmEpiWarps / 4);
 constexpr int kSplitMaxTiles = 320;                      // tiles a split-K launch may have
 constexpr int kSplitMaxRt = 32;                          // and its tile height
 constexpr size_t kSplitAccBytes = size_t(kSplitMaxTiles) * kDigits * kSplitMaxRt * 128 * 4;   // 15.7 MB
-constexpr int kGemmOffScal = 1024;                       // SegScalars[80]
+constexpr int kGemmOffScal = 1024;                       // four floats for each of up to 160 rows
 constexpr int kGemmOffRing = 4096;
 constexpr int kGemmSmem = kGemmOffRing + kGemmRingBytes;
 
 // The digit rows of a launch are laid out [matrix][digit][Rpad][K] with Rpad = R rounded up to 16,
-// whatever tile height the GEMM then picks: a tile that reaches past row R reads the next digit
-// plane (or TMA's zero fill past the end) into accumulator columns that are never stored.
+// whatever tile height the GEMM then picks: a tile that reaches past row Rpad gets TMA's zero fill, and the
+// accumulator columns past row R are never stored.
 inline int gemm_padded_rows(int R) { return (R + 15) / 16 * 16; }
 
 struct GemmSeg {
@@ -206,15 +206,6 @@ __device__ __forceinline__ void tma_operand_4d(uint32_t dst, const CUtensorMap* 
   else tma_load_4d(dst, map, c0, c1, c2, c3, bar);
 }
 
-// 16 consecutive int32 columns of this warp's 32 lanes.
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, int (&v)[16]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
-        "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-      : "r"(taddr)
-      : "memory");
-}
 // 8 consecutive int32 columns of this warp's 32 lanes.
 __device__ __forceinline__ void tmem_ld8(uint32_t taddr, int (&v)[8]) {
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
@@ -271,6 +262,9 @@ inline int gemm_block_tiles(int row_tiles, int rows_tile, int K) {
 // commit) costs about 0.2 us whatever it moves, so small tiles take two chunks per turn where the ring
 // still holds three stages of them, or four in a pair (fewer are slower than twice as many half as large).
 inline int gemm_chunks_per_stage(int chunk_bytes, int nk, bool pair) { return nk >= 2 && (pair ? 4 : 3) * 2 * chunk_bytes <= kGemmRingBytes ? 2 : 1; }
+
+// An accumulator of at most 256 columns has a second buffer.
+inline bool gemm_double_buffered(bool pair, int Rt) { return kDigits * (pair ? 2 * Rt : Rt) <= kGemmAcc1Col; }
 
 // kPair: two CTAs of a cluster work on one tile with tcgen05.mma.cta_group::2 (see the file comment).
 template <bool kPair>
@@ -1004,7 +998,7 @@ __device__ __forceinline__ void rows_prep_long(const RowsPrepParams& P, float* r
 // row needs (fewer registers, more resident CTAs).  256 threads while a row fits, else 512.
 constexpr int kRowsPrepGroupsLn = 4, kRowsPrepGroupsPlain = 8;
 constexpr int rows_prep_min_ctas(int NT, int mode, int G) {
-  return NT == 1024 ? 2 : mode == ROWS_LN ? (NT == 256 ? (G <= 2 ? 5 : G == 3 ? 4 : 3) : (G <= 3 ? 2 : 1))
+  return mode == ROWS_LN ? (NT == 256 ? (G <= 2 ? 5 : G == 3 ? 4 : 3) : (G <= 3 ? 2 : 1))
                          : (NT == 256 ? (G <= 4 ? 5 : 4) : 2);
 }
 
