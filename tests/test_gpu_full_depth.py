@@ -74,7 +74,7 @@ def test_full_depth_unquantised_1b5_against_the_oracle():
 
 def test_full_3b_prompt_of_1024_tokens_against_the_oracle():
     """The 3B shape at full depth, 8 streams x 1024 tokens in sequence mode (tensor-core GEMMs + the
-    chunk-parallel WKV scan over T = 1024): logits after the last token and the final state of two of the
+    WKV scan in chunks of 16 steps): logits after the last token and the final state of two of the
     streams against the oracle's sequence mode (the streams are independent; the oracle needs about half a
     minute per stream on the host)."""
     L, D = SHAPES["3b"]

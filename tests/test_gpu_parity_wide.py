@@ -55,8 +55,8 @@ def test_layer_norm_statistics_with_large_activations(case):
 
 
 def test_chunked_wkv_scan_at_1024_tokens_against_the_oracle():
-    """One block at the 3B width, 8 streams x 1024 tokens in one rows call: the WKV recurrence runs as
-    two passes over 64-step chunks.  time_decay covers the whole U[-5, 3] range of the synthetic
+    """One block at the 3B width, 8 streams x 1024 tokens in one rows call: the WKV recurrence runs
+    in chunks of 16 steps, 16 of them at once.  time_decay covers the whole U[-5, 3] range of the synthetic
     checkpoints.  Logits after the last token and the final state against the oracle's sequence mode."""
     D, V, B, T = 2560, 1024, 8, 1024
     ck = synth_checkpoint(1, D, vocab=V, seed=77)

@@ -166,7 +166,7 @@ def test_rows_path_agrees_with_one_row_path(tiny):
 
 
 def test_rows_long_rows_use_the_chunked_scan_and_agree_with_the_one_row_path(tiny):
-    B, T = 2, 200                                  # > 128 tokens per stream: WKV runs as parallel 64-step chunks
+    B, T = 2, 200                                  # WKV runs as 29 chunks of 7 steps at once
     toks = synth_tokens(B * T, seed=13, vocab=257).reshape(B, T)
     st_rows, st_seq = tiny.empty_batch_state(B), tiny.empty_batch_state(B)
     lg_rows, _ = tiny.forward_batch(toks, st_rows, rows=True)
@@ -260,15 +260,19 @@ def test_rows_path_agrees_with_one_row_path_at_the_1b5_shape():
     model.check_status()
 
 
-@pytest.mark.parametrize("embed", [512, 2048, 4096, 5120])
-def test_row_preparation_gives_the_same_bits_however_rows_are_grouped(embed):
-    """With thousands of rows a preparation CTA walks several consecutive rows for all matrices and keeps the
-    layer norm of a row as the next row's token-shift partner; with few rows there is one CTA per (matrix, row).
-    Six streams of 280 tokens in one call (1680 rows: groups of rows that straddle the stream boundaries)
-    must give exactly the logits and states of the same streams run one per call.  The widths cover every
-    instantiation family: 1, 2 and 4 register groups per thread at 256 threads, 512 threads at 5120 inputs,
-    and for the ffn value input (4 x embed) 256 threads, 512 threads and the rows too long for registers."""
-    model = B200RWKV.synthetic(2, embed, vocab=1000, seed=9, device=DEV)
+@pytest.mark.parametrize("embed,scheme", [(512, "fastquant"), (2048, "fastquant"), (4096, "fastquant"), (5120, "fastquant"),
+                                          (5376, "fastquant"), (8192, "fastquant"),
+                                          (512, "two_axis"), (2048, "two_axis"), (3072, "two_axis"), (4096, "two_axis"), (5120, "two_axis")])
+def test_row_preparation_gives_the_same_bits_however_rows_are_grouped(embed, scheme):
+    """With thousands of rows a preparation CTA walks several consecutive rows and keeps the layer norm of a row as the
+    next row's token-shift partner; with few rows it takes one.  Six streams of 280 tokens in one call (1680 rows:
+    groups of rows that straddle the stream boundaries) must give exactly the logits and states of the same streams
+    run one per call.  Matrices without per-output terms take rows_stream_kernel up to 5120 inputs (one and two groups
+    of inputs per thread) and rows_prep_kernel beyond; two-axis ones need two more sums per row and take
+    rows_prep_kernel (1 to 4 groups at 256 threads, 512 threads at 5120).  The ffn value input (4 x embed) takes
+    rows_stream_kernel at 2048 and 20480 inputs, and rows_prep_kernel with 256 and with 512 threads or the form for
+    rows too long for registers at the others."""
+    model = B200RWKV.synthetic(2, embed, vocab=1000, seed=9, scheme=scheme, device=DEV)
     B, T = 6, 280
     toks = synth_tokens(B * T, seed=44, vocab=1000).reshape(B, T)
     start = model.empty_batch_state(B)
@@ -280,4 +284,22 @@ def test_row_preparation_gives_the_same_bits_however_rows_are_grouped(embed):
         lg = model.forward_rows(toks[b:b + 1], st)
         assert torch.equal(lg[0], lg_all[b]), b
         assert torch.equal(st[0], st_all[b]), b
+    model.check_status()
+
+
+@pytest.mark.parametrize("embed,scheme", [(512, "two_axis"), (2048, "two_axis"), (4096, "two_axis"), (5120, "two_axis"), (5376, "fastquant")])
+def test_rows_path_agrees_with_the_one_row_path_where_rows_prep_kernel_takes_the_layer_norm(embed, scheme):
+    """450 rows in one call (a CTA takes several, begins inside a stream and parks the carries of the stream ends) and
+    57, from carried states; the same tolerance as test_rows_path_agrees_with_the_one_row_path_at_every_width."""
+    model = B200RWKV.synthetic(2, embed, vocab=515, seed=3, scheme=scheme, device=DEV)
+    model.rows_threshold = 1 << 30
+    for T in (19, 150):
+        toks = synth_tokens(3 * T, seed=embed + T, vocab=515).reshape(3, T)
+        start = model.empty_batch_state(3)
+        start[:, :, :2] = torch.randn(start[:, :, :2].shape, device=DEV, generator=torch.Generator(device=DEV).manual_seed(1))
+        st_rows, st_one = start.clone(), start.clone()
+        lg_rows, _ = model.forward_batch(toks, st_rows, rows=True)
+        lg_one, _ = model.forward_batch(toks, st_one, rows=False)
+        assert float((lg_rows - lg_one).abs().max()) < 2e-4 * max(1.0, float(lg_one.abs().max()))
+        assert torch.allclose(st_rows[:, :, :4], st_one[:, :, :4], rtol=1e-3, atol=2e-4)
     model.check_status()

@@ -1,5 +1,6 @@
 """The streaming row preparation where its shape changes: one and two input groups per thread (a ragged second
-one at 4224 inputs), one to five for the ffn value input, CTAs that begin inside a stream."""
+one at 4224 inputs) with the layer norm, two, three and five for plain rows (up to 4096 inputs, up to 6144, beyond
+16384; rows_prep_kernel between), CTAs that begin inside a stream."""
 import pytest
 import torch
 
