@@ -12,8 +12,8 @@
 // and n depends on T alone, so a stream's bits do not depend on how many warps a CTA has.  Longer
 // sequences continue with the carried state.
 // Kept as loops over four steps: with all steps of a warp unrolled and held in registers the kernel took
-// 152 instead of 62 us (8 streams x 512 tokens, 2560 channels; 110 instructions per element, 0.63 issued
-// per clock, the rest waits for L2); requesting the next four steps ahead gained nothing, two at a time
+// 152 instead of 62 us (8 streams x 512 tokens, 2560 channels; 0.65 instructions issued per clock and
+// scheduler, the rest waits for L2); requesting the next four steps ahead gained nothing, two at a time
 // lost 30 %.  The two passes over 64-step chunks that this replaces took 85 us, and 48 instead of 10 us for
 // one stream of 333 tokens at 4096 channels.
 #pragma once

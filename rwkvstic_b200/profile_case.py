@@ -9,7 +9,7 @@ With ``--rows R`` (R > 1) the same matrices are applied to R activation rows thr
 tensor-core path instead (row preparation + ``tile_gemm_kernel``): ``ncu -k regex:tile_gemm``.
 
 With ``--dense bf16|fp16|fp32`` the first matrix of the shape is streamed unquantised
-(``dense_gemv_kernel``), and with ``--sampler`` one row of V logits goes through the typical
+(``dense_gemv_kernel``), and with ``--sampler`` ``--rows`` rows of V logits go through the typical
 sampling kernel (``sample_typical_kernel``).  ``--dense-step bf16|fp16|fp32`` runs --launches
 tokens through the unquantised model of --shape (``dense_rows_kernel``, ``dense_vec_kernel``;
 ``--network LAYERS`` truncates it), graph-replayed, and prints the time per token; with
@@ -55,7 +55,7 @@ def main():
     ap.add_argument("--dense-step", default=None, choices=["bf16", "fp16", "fp32"],
                     help="decode --launches tokens with the unquantised model of --shape in this type")
     ap.add_argument("--dense-rows", action="store_true", help="with --dense-step: --streams x --tokens rows per call through the rows path")
-    ap.add_argument("--sampler", action="store_true", help="typical sampling of one row of V logits")
+    ap.add_argument("--sampler", action="store_true", help="typical sampling of --rows rows of V logits")
     ap.add_argument("--trace", default=None, choices=["chained", "persistent"],
                     help="print the %%globaltimer timeline of one block of a graph-replayed decode step of --shape "
                          "(--network LAYERS blocks, default 4) in this decode mode")
@@ -147,17 +147,17 @@ def main():
     _, D = SHAPES[args.shape]
     if args.sampler:
         g = torch.Generator(device=dev).manual_seed(2)
-        logits = torch.randn(VOCAB, generator=g, device=dev) * 4.0
-        u = torch.rand(args.launches, generator=g, device=dev)
+        logits = torch.randn(args.rows, VOCAB, generator=g, device=dev) * 4.0
+        u = torch.rand(args.launches, args.rows, generator=g, device=dev)
         times = []
         for i in range(args.launches):
             e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
             e0.record()
-            ops.sample_typical(logits, 1.0, 0.95, u=u[i:i + 1])
+            ops.sample_typical(logits, 1.0, 0.95, u=u[i])
             e1.record()
             e1.synchronize()
             times.append(e0.elapsed_time(e1) * 1e3)
-        print(f"typical sampling of {VOCAB} logits, event time per launch (us): " + " ".join(f"{t:.1f}" for t in times))
+        print(f"typical sampling of {args.rows} x {VOCAB} logits, event time per launch (us): " + " ".join(f"{t:.1f}" for t in times))
         return
     if args.dense:
         dt = {"bf16": torch.bfloat16, "fp16": torch.float16, "fp32": torch.float32}[args.dense]
