@@ -97,6 +97,7 @@ struct GemmParams {
   int ksplit;          // 1, 2, 4 or 8 slices (divides K/128; only single-CTA tiles with Rt <= 32)
   int* sk_acc;         // [kSplitMaxTiles][3*Rt][128] int32, zero between launches
   unsigned* sk_count;  // [kSplitMaxTiles] tickets, zero between launches
+  int late_weights;    // the weights may be what the kernel in front of the launch in front wrote: wait before reading them
   int* status;
 };
 
@@ -335,7 +336,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1) tile_gemm_kernel(const __grid
       ld.it = first_item;
       start(ld);
       int early = 0;
-      for (; early < NS && ld.it < nitems_all; ++early, next(ld)) {
+      const int most = P.late_weights ? 0 : NS;
+      for (; early < most && ld.it < nitems_all; ++early, next(ld)) {
         if (elect_one()) {
           if (rank == 0) mbar_arrive_expect_tx(full0 + 8 * early, tx_bytes);
           tma_operand_3d<kPair>(ring0 + uint32_t(early) * stage_bytes, &P.seg[ld.T.seg].wmap, 0, ld.T.n0 + rank * 128, ld.k, full_at + 8 * early);
