@@ -599,7 +599,11 @@ static cudaError_t launch_tile_gemm_as(GemmParams& P, const b200rwkv_matrix* con
 // K = 16384, 16 to 320 rows); they are shared-memory traffic (operands in by TMA, out to the tensor
 // core), which is why a pair, whose CTAs each hold half of the digit rows, needs less per row.  A tile
 // whose accumulator has no second buffer waits 3.6 us for its epilogue; a K slice pays 3 us for its
-// atomics and ticket.
+// atomics and ticket.  Below about ten steps the epilogue bounds a tile, whatever its steps (K = 128, 2 to 8
+// rounds of every form: 1.56 us + 0.0305 a row for a CTA, 1.87 + 0.035 for a pair); without that bound 64-row pair
+// tiles were taken there, up to 20 % slower than single ones (3 x [768 x 768], 512 rows 17.4 -> 16.4 us;
+// 3 x [16384 x 768], 124 rows 35.3 -> 30.5).  Of all forms timed at 107 sizes (K 128 to 20480, 16 to 4096 rows) the
+// one taken is 1.2 % above the fastest on average.
 static void gemm_pick_tile(const GemmParams& P, long long sms, int* pair, int* Rt, int* ksplit) {
   static const double step_single[5] = {0.16, 0.215, 0.26, 0.32, 0.345}, step_pair[5] = {0.18, 0.25, 0.40, 0.45, 0.555};   // Rt = 16, 32, .. 80
   sms = sms > 1 ? sms : 2;
@@ -620,7 +624,9 @@ static void gemm_pick_tile(const GemmParams& P, long long sms, int* pair, int* R
           continue;
         const long long units = pr ? sms / 2 : sms;
         const double rounds = double((tiles * ks + units - 1) / units);
-        const double cost = rounds * (double(nk / ks) * (pr ? step_pair[i] : step_single[i]) + (ks > 1 ? 3.0 : dbuf ? 1.2 : 3.6));
+        const double steps = double(nk / ks) * (pr ? step_pair[i] : step_single[i]) + (ks > 1 ? 3.0 : dbuf ? 1.2 : 3.6);
+        const double epilogue = pr ? 1.87 + 0.035 * rows : 1.56 + 0.0305 * rows;
+        const double cost = rounds * std::max(steps, epilogue);
         if (best == 0.0 || cost < best) { best = cost; *pair = pr; *Rt = rt; *ksplit = ks; }
       }
     }
