@@ -21,9 +21,10 @@
 // over it (maximum, softmax sums, histogram, draw sums with the candidates set aside) run from there.
 // Measured at n = 50277, logits from HBM: 1 row 27 us, 37 rows 38, 74 rows 44, 148 rows 57, 256 rows 102 (two
 // waves of clusters), against 68, 72, 72, 74 and 138 with one CTA of 1024 threads per row and eight passes
-// through L2.  Of these, sums in fp64 per term (conversions go through a slow pipe) and in fixed parts cost 9 us
-// at 256 rows and 1 at 1; parts added up in the order of whatever CTAs a row got would save 5 of the 9, but
-// then the last bit of a row's sums would depend on the number of rows in the call.
+// through L2.  Sums in fp64 per term and in fixed parts are 9 us of it at 256 rows and 1 at 1 row: parts added up
+// in the order of whatever CTAs a row got would save 5 of the 9, but then the last bit of a row's sums would
+// depend on the number of rows in the call; terms built from the bits of the fp32 number instead of converted
+// cost 4 more.
 #pragma once
 
 #include <cooperative_groups.h>
