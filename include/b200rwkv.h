@@ -172,6 +172,9 @@ size_t b200rwkv_decode_workspace_bytes(const b200rwkv_model* m);
  *             first int is the status word the kernels OR error bits into (zero it once).
  * Launches 8*n_layer + 3 kernels (per matrix group one activation-preparation CTA and one
  * streaming GEMV grid) chained by programmatic dependent launch; safe to capture in a CUDA graph.
+ * The first launch is chained to the work in front of the call too, so that steps of a loop overlap: weights and
+ * parameter vectors are read early and must not be written by a kernel right in front that lets its
+ * dependents start early (as this library's do).  The rows and gemv / gemm entry points have no such limit.
  */
 int b200rwkv_decode_step(const b200rwkv_model* m, const int64_t* token, float* state, float* logits,
                          void* workspace, size_t workspace_bytes, void* stream);
